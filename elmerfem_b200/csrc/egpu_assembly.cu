@@ -2,11 +2,13 @@
 //
 // Replaces the bulk element loops of HeatSolve (modules/HeatSolve.src:655-985) and
 // StressSolve (modules/StressSolve.src:815-1072) for linear isotropic diffusion and
-// isotropic elasticity.  One warp computes one element: lanes < ngauss evaluate the
-// geometry of one integration point each (ElementInfo / ElementMetric,
-// ElementDescription.src:2586-3320, 6757-6884) into shared memory, then all lanes form
-// the element matrix entries and add them to precomputed CRS positions.  Elements of one
-// colour share no node, so the scatter needs no atomics; colours run one after another.
+// isotropic elasticity.  Hexahedra: one warp computes four elements on the FP64 matrix
+// instruction.  Tetrahedra and triangles: one warp computes one element; lanes < ngauss
+// evaluate the geometry of one integration point each (ElementInfo / ElementMetric,
+// ElementDescription.src:2586-3320, 6757-6884) into shared memory, then all lanes form the
+// element matrix entries.  Entries are added to precomputed CRS positions.  Elements of one
+// colour share no node, so the scatter needs no atomics; the groups (a range of rows, then a
+// colour) run one after another.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -22,32 +24,6 @@ namespace egpu {
 // nodal basis (elements.def 808 :606-643, 504 :365-404, 303 :155-185)
 template <int CODE>
 struct Ref;
-
-template <>
-struct Ref<808> {
-  static constexpr int NEN = 8, NGP = 8, DIM = 3;
-  __device__ static void gp(int t, double &u, double &v, double &w, double &s) {
-    const double a = 0.57735026918962576451;  // 1/sqrt(3)
-    const int i = t >> 2, j = (t >> 1) & 1, k = t & 1;
-    u = k ? a : -a;
-    v = j ? a : -a;
-    w = i ? a : -a;
-    s = 1.0;
-  }
-  __device__ static void basis(double u, double v, double w, double *N, double (*dN)[3]) {
-    const double nu[8] = {-1, 1, 1, -1, -1, 1, 1, -1};
-    const double nv[8] = {-1, -1, 1, 1, -1, -1, 1, 1};
-    const double nw[8] = {-1, -1, -1, -1, 1, 1, 1, 1};
-#pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      const double a = 1.0 + nu[p] * u, b = 1.0 + nv[p] * v, c = 1.0 + nw[p] * w;
-      N[p] = 0.125 * a * b * c;
-      dN[p][0] = 0.125 * nu[p] * b * c;
-      dN[p][1] = 0.125 * nv[p] * a * c;
-      dN[p][2] = 0.125 * nw[p] * a * b;
-    }
-  }
-};
 
 template <>
 struct Ref<504> {
@@ -174,7 +150,295 @@ __device__ bool gp_geometry(int t, const double (*X)[3], int cdim, double *N, do
   return true;
 }
 
+// FP64 matrix instruction D = A B + D on one 8x8 tile (A 8x4 row-major, B 4x8 column-major):
+// lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) + {0, 1}].
+__device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
 constexpr int ASM_WARPS = 8;
+constexpr long long ASM_RANGE_BYTES = 40LL << 20;  // Values of one row range (see egpu_assembly_bind)
+
+// ------------------------------------------------------------------------------------
+// Hexahedra (808), four elements per warp.
+//
+// The element matrix is a contraction over the integration points: with the gradients
+// G_t(p, i) = dN_p/dx_i at point t, Poisson's K = sum_(t,i) (w_t G_t(p,i)) G_t(q,i) is an
+// 8x24 by 24x8 product, and elasticity's M_ij = sum_t (s_t G_t(p,i)) G_t(q,j) nine 8x8x8
+// ones.  Both run on the FP64 matrix instruction, whose fragments put node p = lane / 4 and
+// point t = lane % 4 (+ 4) on a lane: the same value is the A operand (times the weight)
+// and the B operand, so a lane needs the gradients of one node at two points only, and forms
+// them itself from the points' 3x3 geometry factors L_t (gradient = L_t dN/dxi).
+//   1. lane = (element, node): node ids, coordinates and material, staged in shared memory
+//   2. lane = (element, point): Jacobian, metric, L_t and the weights, into shared memory
+//      (all 32 lanes busy; one element per warp left 24 of them idle)
+//   3. per element: two gradients per lane, six (Poisson) or eighteen (elasticity) matrix
+//      instructions, and the accumulators are exactly the lane's CRS entries (two columns)
+// The CRS positions and the values they hold are loaded before step 2, so their latency is
+// covered by it.  Elements of a group share no node, so the preloaded values are current.
+constexpr int HEX_EPW = 4;       // elements per warp
+constexpr int HEX_XS = 25;       // doubles per element of staged coordinates (24 + 1: no bank conflicts)
+constexpr int HEX_LS = 12;       // doubles per point: L (9), weight, load weight, pad
+
+struct HexShared {
+  double X[HEX_EPW * HEX_XS];
+  double kn[32], ln[32];
+  double2 L[32 * HEX_LS / 2];
+};
+
+// reference coordinates of node p and point t as sign bits (u, v, w); 1 = +
+__device__ __forceinline__ int hex_node_bits(int p) { return ((0x66 >> p) & 1) | (((0xCC >> p) & 1) << 1) | ((p >> 2) << 2); }
+
+// dN_p/dxi at point t (elements.def 808 :606-643, 2-point Gauss per direction)
+__device__ __forceinline__ void hex_dN(int p, int t, double &d0, double &d1, double &d2) {
+  const double g = 0.57735026918962576451;  // 1/sqrt(3)
+  const int pb = hex_node_bits(p), x = pb ^ t;
+  const double a = (x & 1) ? 1.0 - g : 1.0 + g, b = (x & 2) ? 1.0 - g : 1.0 + g, c = (x & 4) ? 1.0 - g : 1.0 + g;
+  d0 = ((pb & 1) ? 0.125 : -0.125) * b * c;
+  d1 = ((pb & 2) ? 0.125 : -0.125) * a * c;
+  d2 = ((pb & 4) ? 0.125 : -0.125) * a * b;
+}
+__device__ __forceinline__ double hex_N(int p, int t) {
+  const double g = 0.57735026918962576451;
+  const int x = hex_node_bits(p) ^ t;
+  const double a = (x & 1) ? 1.0 - g : 1.0 + g, b = (x & 2) ? 1.0 - g : 1.0 + g, c = (x & 4) ? 1.0 - g : 1.0 + g;
+  return 0.125 * a * b * c;
+}
+
+// step 2 for lane (el, t): L_t = dx GI with GI the inverse metric (ElementMetric), and
+// s = sqrt(detG); a degenerate element (DetG <= TINY) gets L = 0, s = 0
+__device__ __forceinline__ double hex_point(const double *X, int t, int cdim, double (&L)[3][3]) {
+  double dx[3][3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dx[c][i] = 0.0;
+#pragma unroll
+  for (int p = 0; p < 8; ++p) {
+    double d0, d1, d2;
+    hex_dN(p, t, d0, d1, d2);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double x = X[3 * p + c];
+      dx[c][0] += x * d0;
+      dx[c][1] += x * d1;
+      dx[c][2] += x * d2;
+    }
+  }
+  double G[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = i; j < 3; ++j) {
+      double acc = dx[0][i] * dx[0][j] + dx[1][i] * dx[1][j];
+      if (cdim > 2) acc += dx[2][i] * dx[2][j];
+      G[i][j] = acc;
+      G[j][i] = acc;
+    }
+  const double detG = G[0][0] * (G[1][1] * G[2][2] - G[1][2] * G[2][1]) + G[0][1] * (G[1][2] * G[2][0] - G[1][0] * G[2][2]) +
+                      G[0][2] * (G[1][0] * G[2][1] - G[1][1] * G[2][0]);
+  const bool ok = detG > EGPU_TINY_DP;
+  const double q = ok ? 1.0 / detG : 0.0;
+  double GI[3][3];
+  GI[0][0] = q * (G[1][1] * G[2][2] - G[2][1] * G[1][2]);
+  GI[1][0] = -q * (G[1][0] * G[2][2] - G[2][0] * G[1][2]);
+  GI[2][0] = q * (G[1][0] * G[2][1] - G[2][0] * G[1][1]);
+  GI[1][1] = q * (G[0][0] * G[2][2] - G[2][0] * G[0][2]);
+  GI[2][1] = -q * (G[0][0] * G[2][1] - G[2][0] * G[0][1]);
+  GI[2][2] = q * (G[0][0] * G[1][1] - G[1][0] * G[0][1]);
+  GI[0][1] = GI[1][0];
+  GI[0][2] = GI[2][0];
+  GI[1][2] = GI[2][1];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      L[i][j] = i < cdim ? dx[i][0] * GI[0][j] + dx[i][1] * GI[1][j] + dx[i][2] * GI[2][j] : 0.0;
+  return ok ? sqrt(detG) : 0.0;
+}
+
+// gradient of the lane's node at one point: row i of L_t times dN/dxi; returns the weight
+__device__ __forceinline__ double hex_grad(const double2 *L, double d0, double d1, double d2, double (&g)[3]) {
+  const double2 l0 = L[0], l1 = L[1], l2 = L[2], l3 = L[3], l4 = L[4];
+  g[0] = d0 * l0.x + d1 * l0.y + d2 * l1.x;
+  g[1] = d0 * l1.y + d1 * l2.x + d2 * l2.y;
+  g[2] = d0 * l3.x + d1 * l3.y + d2 * l4.x;
+  return l4.y;
+}
+
+__device__ __forceinline__ void hex_store_point(double2 *L, const double (&l)[3][3], double w, double f) {
+  L[0] = make_double2(l[0][0], l[0][1]);
+  L[1] = make_double2(l[0][2], l[1][0]);
+  L[2] = make_double2(l[1][1], l[1][2]);
+  L[3] = make_double2(l[2][0], l[2][1]);
+  L[4] = make_double2(l[2][2], w);
+  L[5] = make_double2(f, 0.0);
+}
+
+// Diffusion on 808: K_pq = sum_t s_t k_t dN_q.dN_p, f_p = sum_t s_t (sum_m load_m N_m) N_p
+// (DiffuseConvectiveAnisotropic.src:334-344, 515-561, 569-612)
+__global__ void __launch_bounds__(ASM_WARPS * 32, 2) k_assemble_poisson_hex(
+    int ne, const int *__restrict__ elist, const int *__restrict__ enodes, const double *__restrict__ xyz,
+    int cdim, const double *__restrict__ elem_k, const double *__restrict__ nodal_k,
+    const double *__restrict__ load, const int *__restrict__ perm, const int *__restrict__ slots,
+    double *__restrict__ values, double *__restrict__ rhs) {
+  __shared__ __align__(16) HexShared sh_all[ASM_WARPS];
+  HexShared &sh = sh_all[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int w0 = (blockIdx.x * ASM_WARPS + (threadIdx.x >> 5)) * HEX_EPW;
+  if (w0 >= ne) return;
+  const int el = lane >> 3, nd = lane & 7;
+  const bool have = w0 + el < ne;
+  const int e = have ? elist[w0 + el] : 0;
+  const int node = have ? enodes[(size_t)e * 8 + nd] : 0;
+  // this lane's CRS positions (node lane/4's row, two columns) and their present values
+  int2 sl[HEX_EPW];
+  double2 old[HEX_EPW];
+#pragma unroll
+  for (int j = 0; j < HEX_EPW; ++j) {
+    const int ej = __shfl_sync(0xffffffffu, e, 8 * j);
+    sl[j] = w0 + j < ne ? __ldcs(reinterpret_cast<const int2 *>(slots + (size_t)ej * 64) + lane) : make_int2(-1, -1);
+  }
+  sh.kn[lane] = !have ? 0.0 : elem_k ? elem_k[e] : (nodal_k ? nodal_k[node] : 1.0);
+  sh.ln[lane] = have && load ? load[node] : 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) sh.X[el * HEX_XS + 3 * nd + c] = have ? xyz[(size_t)node * 3 + c] : 0.0;
+#pragma unroll
+  for (int j = 0; j < HEX_EPW; ++j) {
+    old[j].x = sl[j].x >= 0 ? values[sl[j].x] : 0.0;
+    old[j].y = sl[j].y >= 0 ? values[sl[j].y] : 0.0;
+  }
+  __syncwarp();
+  {
+    double L[3][3];
+    const double s = hex_point(sh.X + el * HEX_XS, nd, cdim, L);
+    double kk = 0.0, ff = 0.0;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const double N = hex_N(p, nd);
+      kk += sh.kn[8 * el + p] * N;
+      ff += sh.ln[8 * el + p] * N;
+    }
+    hex_store_point(sh.L + lane * (HEX_LS / 2), L, s * kk, s * ff);
+  }
+  __syncwarp();
+  const int p = lane >> 2, kq = lane & 3;
+  double d1[3], d2[3];
+  hex_dN(p, kq, d1[0], d1[1], d1[2]);
+  hex_dN(p, kq + 4, d2[0], d2[1], d2[2]);
+#pragma unroll
+  for (int j = 0; j < HEX_EPW; ++j) {
+    double g[3], c0 = 0.0, c1 = 0.0;
+    double wt = hex_grad(sh.L + (8 * j + kq) * (HEX_LS / 2), d1[0], d1[1], d1[2], g);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dmma_8x8x4(c0, c1, wt * g[i], g[i]);
+    wt = hex_grad(sh.L + (8 * j + kq + 4) * (HEX_LS / 2), d2[0], d2[1], d2[2], g);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dmma_8x8x4(c0, c1, wt * g[i], g[i]);
+    if (sl[j].x >= 0) values[sl[j].x] = old[j].x + c0;
+    if (sl[j].y >= 0) values[sl[j].y] = old[j].y + c1;
+  }
+  if (load && have) {
+    double F = 0.0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) F += sh.L[(8 * el + t) * (HEX_LS / 2) + 5].x * hex_N(nd, t);
+    const int r = perm[node];
+    if (r >= 0) rhs[r] += F;
+  }
+}
+
+// Isotropic elasticity on 808 (see k_assemble_elastic for the form of K): the nine 8x8
+// matrices M_ij of a node pair end on one lane, which combines them,
+//   K_(p,i),(q,j) = c12 M_ij + c44 (M_ji + delta_ij (M_00 + M_11 + M_22)).
+__global__ void __launch_bounds__(ASM_WARPS * 32, 2) k_assemble_elastic_hex(
+    int ne, const int *__restrict__ elist, const int *__restrict__ enodes, const double *__restrict__ xyz,
+    double c12, double c44, double bf0, double bf1, double bf2, const int *__restrict__ perm,
+    const int *__restrict__ slots, double *__restrict__ values, double *__restrict__ rhs) {
+  __shared__ __align__(16) HexShared sh_all[ASM_WARPS];
+  HexShared &sh = sh_all[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int w0 = (blockIdx.x * ASM_WARPS + (threadIdx.x >> 5)) * HEX_EPW;
+  if (w0 >= ne) return;
+  const int el = lane >> 3, nd = lane & 7;
+  const bool have = w0 + el < ne;
+  const int e = have ? elist[w0 + el] : 0;
+  const int node = have ? enodes[(size_t)e * 8 + nd] : 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) sh.X[el * HEX_XS + 3 * nd + c] = have ? xyz[(size_t)node * 3 + c] : 0.0;
+  __syncwarp();
+  {
+    double L[3][3];
+    const double s = hex_point(sh.X + el * HEX_XS, nd, 3, L);
+    double sn = 0.0;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) sn += hex_N(p, nd);
+    hex_store_point(sh.L + lane * (HEX_LS / 2), L, s, s * sn);
+  }
+  __syncwarp();
+  const int p = lane >> 2, kq = lane & 3;
+  double d1[3], d2[3];
+  hex_dN(p, kq, d1[0], d1[1], d1[2]);
+  hex_dN(p, kq + 4, d2[0], d2[1], d2[2]);
+  for (int j = 0; j < HEX_EPW && w0 + j < ne; ++j) {
+    const int ej = __shfl_sync(0xffffffffu, e, 8 * j);
+    // row (p, i): six consecutive positions, columns (q, q + 1) x 3 DOFs
+    const int *sb = slots + (size_t)ej * 576 + 72 * p + 6 * kq;
+    int2 sl[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int h = 0; h < 3; ++h) sl[i][h] = __ldcs(reinterpret_cast<const int2 *>(sb + 24 * i) + h);
+    double g1[3], g2[3];
+    const double w1 = hex_grad(sh.L + (8 * j + kq) * (HEX_LS / 2), d1[0], d1[1], d1[2], g1);
+    const double w2 = hex_grad(sh.L + (8 * j + kq + 4) * (HEX_LS / 2), d2[0], d2[1], d2[2], g2);
+    double M[3][3][2];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        M[i][c][0] = M[i][c][1] = 0.0;
+        dmma_8x8x4(M[i][c][0], M[i][c][1], w1 * g1[i], g1[c]);
+        dmma_8x8x4(M[i][c][0], M[i][c][1], w2 * g2[i], g2[c]);
+      }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      // entry (q, c) of the row sits at 3 q + c of its six
+      double old[6];
+      int pos[6];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        pos[2 * h] = sl[i][h].x;
+        pos[2 * h + 1] = sl[i][h].y;
+      }
+#pragma unroll
+      for (int t = 0; t < 6; ++t) old[t] = pos[t] >= 0 ? values[pos[t]] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double tr = M[0][0][q] + M[1][1][q] + M[2][2][q];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          double v = c12 * M[i][c][q] + c44 * M[c][i][q];
+          if (i == c) v += c44 * tr;
+          if (pos[3 * q + c] >= 0) values[pos[3 * q + c]] = old[3 * q + c] + v;
+        }
+      }
+    }
+  }
+  if (have) {
+    double F = 0.0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) F += sh.L[(8 * el + t) * (HEX_LS / 2) + 5].x * hex_N(nd, t);
+    const int r = perm[node];
+    if (r >= 0) {
+      rhs[3 * r] += bf0 * F;
+      rhs[3 * r + 1] += bf1 * F;
+      rhs[3 * r + 2] += bf2 * F;
+    }
+  }
+}
+
 
 // Diffusion: K_pq = sum_t s_t k_t dN_q.dN_p, f_p = sum_t s_t (sum_m load_m N_m) N_p
 // (DiffuseConvectiveAnisotropic.src:334-344, 515-561, 569-612)
@@ -370,32 +634,57 @@ __global__ void k_fill_zero(double *p, long long n) {
 // DefaultDirichletBCs (DefUtils.src:3530-4031) on the whole matrix in one pass:
 // scale without rhs normalisation, constrained rows -> zero row, unit diagonal,
 // b = val/D (SolverUtils.src:2465-2473), or symmetric elimination (CRS_SetSymmDirichlet,
-// CRSMatrix.src:674-740), then back-scaling.  One thread per row keeps the reference's
-// per-row order of right-hand-side updates.
+// CRSMatrix.src:674-740), then back-scaling.  Eight lanes per row, so a row's values and
+// columns are read and written as whole sectors; the right-hand side takes the constrained
+// columns' terms in column order, as the reference does.
 __global__ void k_dirichlet(int n, const int *__restrict__ rows, const int *__restrict__ cols,
                             const int *__restrict__ diag, double *__restrict__ values, double *__restrict__ rhs,
                             const double *__restrict__ D, const unsigned char *__restrict__ cflag,
                             const double *__restrict__ cval, int symmetric) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double di = D[i];
-    double bi = rhs[i] * di;
-    if (cflag[i]) {
-      for (int k = rows[i]; k < rows[i + 1]; ++k) values[k] = 0.0;
-      values[diag[i]] = 1.0 / (di * di);
+  const int lane = threadIdx.x & 7, sub = threadIdx.x & 24;
+  const int stride = (gridDim.x * blockDim.x) >> 3;
+  // the four rows of a warp run in step, so the collectives below are whole-warp ones
+  for (int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; i0 < n; i0 += stride) {
+    const int i = i0 + (sub >> 3);
+    const bool on = i < n;
+    const double di = on ? D[i] : 1.0;
+    double bi = on ? rhs[i] * di : 0.0;
+    const int beg = on ? rows[i] : 0, end = on ? rows[i + 1] : 0;
+    const bool fixed = on && cflag[i];
+    const int nch = __reduce_max_sync(0xffffffffu, fixed ? 0 : (end - beg + 7) >> 3);
+    if (fixed) {
+      const int dg = diag[i];
+      for (int k = beg + lane; k < end; k += 8) values[k] = k == dg ? 1.0 / (di * di) : 0.0;
       bi = cval[i] / di;
-    } else {
-      for (int k = rows[i]; k < rows[i + 1]; ++k) {
+    }
+#pragma unroll 4
+    for (int ch = 0; ch < nch; ++ch) {
+      const int k = beg + 8 * ch + lane;
+      double term = 0.0;
+      bool con = false;
+      if (!fixed && k < end) {
         const int c = cols[k];
-        const double dd = di * D[c];
+        const double dc = D[c], dd = di * dc;
         double v = values[k] * dd;
         if (symmetric && cflag[c]) {
-          bi = bi - v * (cval[c] / D[c]);
+          con = true;
+          term = v * (cval[c] / dc);
           v = 0.0;
         }
         values[k] = v / dd;
       }
+      if (symmetric) {
+        const unsigned any = __ballot_sync(0xffffffffu, con);
+        if (any) {  // constrained neighbours are rare: the terms in column order, row by row
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const double t = __shfl_sync(0xffffffffu, term, sub + q);
+            if ((any >> (sub + q)) & 1u) bi = bi - t;
+          }
+        }
+      }
     }
-    rhs[i] = bi / di * 1.0;
+    if (on && lane == 0) rhs[i] = bi / di * 1.0;
   }
 }
 
@@ -463,11 +752,27 @@ extern "C" int egpu_assembly_bind(egpu_mat *A, int nnodes, const double *xyz, in
   }
   std::vector<int> color_of;
   const int ncol = egpu_color_elements(nnodes, nelem, nen, elem_nodes, color_of);
-  S.color_ptr.assign(ncol + 1, 0);
-  for (int e = 0; e < nelem; ++e) S.color_ptr[color_of[e] + 1]++;
-  for (int c = 0; c < ncol; ++c) S.color_ptr[c + 1] += S.color_ptr[c];
+  // Groups of elements assembled in one launch: a range of matrix rows, then a colour.  Every
+  // colour touches every row, so running each colour over the whole mesh would stream Values
+  // through HBM once per colour; a range whose Values fit in L2 (ASM_RANGE_BYTES of the 126 MB)
+  // is read and written there once for all its colours.
+  const long long nrange = std::max(1LL, (A->nnz * (long long)sizeof(double) + ASM_RANGE_BYTES / 2) / ASM_RANGE_BYTES);
+  const int nrows = A->n / dofs;
+  std::vector<int> group_of(nelem);
+  for (int e = 0; e < nelem; ++e) {
+    int lo = nrows - 1;
+    for (int k = 0; k < nen; ++k) {
+      const int r = p0[en0[(size_t)e * nen + k]];
+      if (r >= 0) lo = std::min(lo, r);
+    }
+    group_of[e] = (int)((long long)std::max(lo, 0) * nrange / std::max(1, nrows)) * ncol + color_of[e];
+  }
+  const int ngroup = (int)nrange * ncol;
+  S.color_ptr.assign(ngroup + 1, 0);
+  for (int e = 0; e < nelem; ++e) S.color_ptr[group_of[e] + 1]++;
+  for (int c = 0; c < ngroup; ++c) S.color_ptr[c + 1] += S.color_ptr[c];
   std::vector<int> grouped(nelem), fill(S.color_ptr.begin(), S.color_ptr.end() - 1);
-  for (int e = 0; e < nelem; ++e) grouped[fill[color_of[e]]++] = e;
+  for (int e = 0; e < nelem; ++e) grouped[fill[group_of[e]]++] = e;
   const int nd = nen * dofs;
   EGPU_CUDA_TRY(ctx, S.xyz.alloc((size_t)nnodes * 3));
   EGPU_CUDA_TRY(ctx, S.elem_nodes.alloc(en0.size()));
@@ -526,7 +831,8 @@ extern "C" int egpu_assemble_poisson(egpu_mat *A, const double *elem_k, const do
                                                                      dk.p, dn.p, dl.p, S.perm.p, S.slots.p,    \
                                                                      A->values.p, A->rhs.p)
     if (S.code == 808)
-      EGPU_ASM(808);
+      k_assemble_poisson_hex<<<(ne + ASM_WARPS * HEX_EPW - 1) / (ASM_WARPS * HEX_EPW), ASM_WARPS * 32, 0, ctx->stream>>>(
+          ne, el, S.elem_nodes.p, S.xyz.p, S.cdim, dk.p, dn.p, dl.p, S.perm.p, S.slots.p, A->values.p, A->rhs.p);
     else if (S.code == 504)
       EGPU_ASM(504);
     else
@@ -559,7 +865,7 @@ extern "C" int egpu_assemble_elastic(egpu_mat *A, double young, double poisson, 
     const int *el = S.color_elems.p + S.color_ptr[c];
     const int grid = (ne + ASM_WARPS - 1) / ASM_WARPS;
     if (S.code == 808)
-      k_assemble_elastic<808><<<grid, ASM_WARPS * 32, 0, ctx->stream>>>(ne, el, S.elem_nodes.p, S.xyz.p, c12, c44, bf[0],
+      k_assemble_elastic_hex<<<(ne + ASM_WARPS * HEX_EPW - 1) / (ASM_WARPS * HEX_EPW), ASM_WARPS * 32, 0, ctx->stream>>>(ne, el, S.elem_nodes.p, S.xyz.p, c12, c44, bf[0],
                                                                         bf[1], bf[2], S.perm.p, S.slots.p, A->values.p,
                                                                         A->rhs.p);
     else
@@ -602,7 +908,7 @@ extern "C" int egpu_dirichlet(egpu_mat *A, int ncon, const int *con_rows, const 
   }
   // Linear System Dirichlet Scaling defaults to Linear System Scaling = True
   k_dirichlet_scale_diag<<<grid_of(ctx, n), 256, 0, ctx->stream>>>(n, A->rows.p, A->diag.p, A->values.p, D.p);
-  k_dirichlet<<<grid_of(ctx, n), 256, 0, ctx->stream>>>(n, A->rows.p, A->cols.p, A->diag.p, A->values.p, A->rhs.p, D.p,
+  k_dirichlet<<<grid_of(ctx, (long long)n * 8), 256, 0, ctx->stream>>>(n, A->rows.p, A->cols.p, A->diag.p, A->values.p, A->rhs.p, D.p,
                                                         cflag.p, cval.p, symmetric);
   ctx->launches += 2;
   int herr = 0;
