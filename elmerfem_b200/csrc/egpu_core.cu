@@ -10,7 +10,7 @@
 #include <numeric>
 
 #include "egpu_internal.cuh"
-#include "egpu_krylov.cuh"
+#include "egpu_krylov_launch.cuh"
 #include "egpu_solve.h"
 
 using namespace egpu;
@@ -395,7 +395,7 @@ static int grid_for(const egpu_ctx *ctx, long long work, int block = 256) {
 static void build_levels(int n, const std::vector<int> &rows, const std::vector<int> &cols,
                          const std::vector<int> &diag, std::vector<int> &lower,
                          std::vector<int> &upper, int &nlow, int &nup, int &maxl, int &maxu,
-                         int &maxw) {
+                         int &maxw, std::vector<int> &lev_lo, std::vector<int> &lev_up) {
   maxw = 0;
   std::vector<int> lev(n, 0);
   nlow = 0;
@@ -414,6 +414,7 @@ static void build_levels(int n, const std::vector<int> &rows, const std::vector<
   for (int l = 0; l < nlow; ++l) maxw = std::max(maxw, cnt[l + 1] - cnt[l]);
   lower.assign(n, 0);
   for (int i = 0; i < n; ++i) lower[cnt[lev[i]]++] = i;
+  lev_lo = lev;
   nup = 0;
   for (int i = n - 1; i >= 0; --i) {
     int l = 0;
@@ -428,6 +429,7 @@ static void build_levels(int n, const std::vector<int> &rows, const std::vector<
   for (int l = 0; l < nup; ++l) maxw = std::max(maxw, cnt[l + 1] - cnt[l]);
   upper.assign(n, 0);
   for (int i = n - 1; i >= 0; --i) upper[cnt[lev[i]]++] = i;
+  lev_up.swap(lev);
 }
 
 // Node blocks: the largest bs <= TRI_BS_MAX dividing n such that every aligned group of bs
@@ -464,7 +466,7 @@ static int node_block_size(int n, const std::vector<int> &rows, const std::vecto
 // by level, rows ascending inside; upper: rows descending inside).  maxw counts rows.
 static void build_block_levels(int n, int bs, const std::vector<int> &rows, const std::vector<int> &cols,
                                const std::vector<int> &diag, std::vector<int> &lower, std::vector<int> &upper,
-                               int &nlow, int &nup, int &maxw) {
+                               int &nlow, int &nup, int &maxw, std::vector<int> &lev_lo, std::vector<int> &lev_up) {
   const int nb = n / bs;
   std::vector<int> lev(nb, 0);
   nlow = nup = maxw = 0;
@@ -485,6 +487,7 @@ static void build_block_levels(int n, int bs, const std::vector<int> &rows, cons
     const int q = cnt[lev[m]]++;
     for (int k = 0; k < bs; ++k) lower[q * bs + k] = m * bs + k;
   }
+  lev_lo = lev;
   for (int m = nb - 1; m >= 0; --m) {
     int l = 0;
     for (int i = m * bs; i < (m + 1) * bs; ++i)
@@ -502,28 +505,7 @@ static void build_block_levels(int n, int bs, const std::vector<int> &rows, cons
     const int q = cnt[lev[m]]++;
     for (int k = 0; k < bs; ++k) upper[q * bs + k] = m * bs + bs - 1 - k;
   }
-}
-
-// occupancy-sized cooperative launch
-template <typename K, typename Args>
-static int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, size_t smem = 0) {
-  int bps = 0;
-  if (smem > 48 * 1024)
-    EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
-  EGPU_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, EGPU_KBLOCK, smem));
-  if (bps < 1) {
-    egpu_set_error(ctx, "persistent kernel does not fit on an SM");
-    return EGPU_ERR_CUDA;
-  }
-  bps = std::min(bps, 2048 / EGPU_KBLOCK);
-  int grid = ctx->num_sms * bps;
-  if (grid_out) *grid_out = grid;
-  void *kargs[] = {&args};
-  EGPU_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(EGPU_KBLOCK),
-                                                 kargs, smem, ctx->stream));
-  ctx->launches++;
-  return EGPU_OK;
+  lev_up.swap(lev);
 }
 
 // lanes per row of the standalone CRS SpMV (egpu_mv)
@@ -716,6 +698,17 @@ static void view_tri(egpu_mat *A, const egpu_mat *proto) {
       T.cta_sr[v] = P.cta_sr[v];
       T.cta_smem[v] = P.cta_smem[v];
     }
+    T.rg_rows = P.rg_rows;
+    T.rg_ext = P.rg_ext;
+    T.rg_g = P.rg_g;
+    T.rg_k = P.rg_k;
+    T.rg_nt = P.rg_nt;
+    for (int v = 0; v < 2; ++v) {
+      T.rg_ok[v] = P.rg_ok[v];
+      T.rg_stage[v] = P.rg_stage[v];
+    }
+    T.rg_lo.view(P.rg_lo);
+    T.rg_up.view(P.rg_up);
     T.cta_rs = P.cta_rs;
     T.pos_lo.view(P.pos_lo);
     T.pos_up.view(P.pos_up);
@@ -758,19 +751,21 @@ int ensure_tri_schedule(egpu_mat *A) {
       egpu_set_error(ctx, "ILU0 needs a stored diagonal in every row");
       return EGPU_ERR_ARG;
     }
-  std::vector<int> lo, up;
+  std::vector<int> lo, up, lev_lo, lev_up;
   build_levels(n, rows, cols, diag, lo, up, A->tri.lower_levels, A->tri.upper_levels, A->tri.max_lower,
-               A->tri.max_upper, A->tri.max_width);
+               A->tri.max_upper, A->tri.max_width, lev_lo, lev_up);
   A->tri.bs = 1;
   {
     const int bs = node_block_size(n, rows, cols, diag);
     if (bs > 1) {
-      std::vector<int> blo, bup;
+      std::vector<int> blo, bup, blev_lo, blev_up;
       int bl = 0, bu = 0, bw = 0;
-      build_block_levels(n, bs, rows, cols, diag, blo, bup, bl, bu, bw);
+      build_block_levels(n, bs, rows, cols, diag, blo, bup, bl, bu, bw, blev_lo, blev_up);
       if (tri_prefer_node_blocks(A->tri.lower_levels, A->tri.upper_levels, bl, bu, n)) {
         lo.swap(blo);
         up.swap(bup);
+        lev_lo.swap(blev_lo);
+        lev_up.swap(blev_up);
         A->tri.bs = bs;
         A->tri.lower_levels = bl;
         A->tri.upper_levels = bu;
@@ -836,6 +831,8 @@ int ensure_tri_schedule(egpu_mat *A) {
       T.cta_ok[0] = T.cta_ok[1] = false;
     }
   }
+  const int rc = build_range_schedule(A, rows, cols, diag, lev_lo, lev_up);
+  if (rc) return rc;
   A->tri_built = true;
   return EGPU_OK;
 }
@@ -914,6 +911,7 @@ static int ilu_pack(egpu_mat *A) {
       A->up_dinv.p, A->lo_vals32.p, A->up_vals32.p, A->up_dinv32.p);
   ctx->launches++;
   EGPU_CUDA_TRY(ctx, cudaGetLastError());
+  A->rg_packed[0] = A->rg_packed[1] = false;
   const int rc = cta_fill_values(A);
   if (rc) return rc;
   A->ilu_valid = true;
@@ -996,6 +994,15 @@ static void set_tri_vals(KArgs<float> &a, const egpu_mat *A) {
   a.cup.vals = A->cta_up_vals32.p;
 }
 
+static void set_range(RangeTri &r, const RangeTriDev &d, const DevBuf<unsigned char> &rec, int v) {
+  r.lev_ptr = d.lev_ptr.p;
+  r.offset = d.offset[v].p;
+  r.rec = rec.p;
+  r.slot = d.slot.p;
+  r.ext_ptr = d.ext_ptr.p;
+  r.ext = d.ext.p;
+}
+
 template <typename VT>
 static void set_tri(KArgs<VT> &a, const egpu_mat *A) {
   a.lower_order = A->tri.lower_order.p;
@@ -1008,7 +1015,15 @@ static void set_tri(KArgs<VT> &a, const egpu_mat *A) {
   // level-synchronous single-block solves when the cost estimate prefers them
   const TriSchedule &T = A->tri;
   const int v = sizeof(VT) == 8 ? 0 : 1;
-  a.tri_cta = cta_use(A, v) ? 1 : 0;
+  a.rg_rows = range_use(A, v) && A->rg_packed[v] ? T.rg_rows : 0;
+  a.rg_ext = T.rg_ext;
+  a.rg_lg = T.rg_g == 8 ? 3 : T.rg_g / 2;
+  a.rg_nt = T.rg_nt;
+  a.rg_stage = T.rg_stage[v];
+  a.idiag = A->ilu_diag.p;
+  set_range(a.rlo, T.rg_lo, A->rg_lo_rec[v], v);
+  set_range(a.rup, T.rg_up, A->rg_up_rec[v], v);
+  a.tri_cta = !a.rg_rows && cta_use(A, v) ? 1 : 0;
   a.cta_pd = T.cta_pd[v];
   a.cta_rs = T.cta_rs;
   a.cta_sb = T.cta_sb[v];
@@ -1049,47 +1064,20 @@ static int tri_per_block(const egpu_mat *A, int lpr, int grid, int block = EGPU_
   return std::max(1, std::min(per_block_max, (want + grid - 1) / grid));
 }
 
-// One warp per row in the sync-free triangular solves: rows that depend on each other
-// never share a warp, so no lane spins while a diverged lane of its own warp has to
-// produce the value it waits for.
-constexpr int TRI_TS = 32;
-
 template <typename VT>
 static int run_krylov(egpu_mat *A, const KArgs<VT> &a0, int method, bool offs) {
   egpu_ctx *ctx = A->ctx;
   KArgs<VT> a = a0;
   a.tri_per_block = tri_per_block(A, TRI_TS, ctx->num_sms);
-  if (a.precond != EGPU_PREC_ILU0) a.tri_cta = 0;
-  const size_t smem = a.tri_cta ? A->tri.cta_smem[sizeof(VT) == 8 ? 0 : 1] : 0;
-  // the instantiation with the level-synchronous solves only when this matrix uses them
-  const bool cta = a.tri_cta != 0;
-  if (method == EGPU_CG) {
-    if (cta) {
-      if (offs) return launch_coop(ctx, cg_kernel<VT, TRI_TS, true, true>, a, nullptr, smem);
-      return launch_coop(ctx, cg_kernel<VT, TRI_TS, false, true>, a, nullptr, smem);
-    }
-    if (offs) return launch_coop(ctx, cg_kernel<VT, TRI_TS, true, false>, a, nullptr, smem);
-    return launch_coop(ctx, cg_kernel<VT, TRI_TS, false, false>, a, nullptr, smem);
-  }
+  if (a.precond != EGPU_PREC_ILU0) a.tri_cta = a.rg_rows = 0;
+  const size_t smem = a.tri_cta ? A->tri.cta_smem[sizeof(VT) == 8 ? 0 : 1] : a.rg_rows ? range_smem_bytes<VT>(a.rg_rows, a.rg_ext, a.rg_stage) : 0;
+  // the instantiation of the form this matrix uses
+  const int form = a.tri_cta ? TRI_CTA : a.rg_rows ? (A->tri.rg_k == 10 ? TRI_RANGE10 : TRI_RANGE7) : TRI_SYNCFREE;
+  if (method == EGPU_CG) return launch_cg(ctx, a, offs, form, smem);
   if constexpr (sizeof(VT) == 8) {
-    if (method == EGPU_GCR)
-      return cta ? launch_coop(ctx, gcr_kernel<TRI_TS, true>, a, nullptr, smem)
-                 : launch_coop(ctx, gcr_kernel<TRI_TS, false>, a, nullptr, smem);
-    if (method == EGPU_BICGSTABL)
-      return cta ? launch_coop(ctx, bicgstabl_kernel<TRI_TS, true>, a, nullptr, smem)
-                 : launch_coop(ctx, bicgstabl_kernel<TRI_TS, false>, a, nullptr, smem);
+    if (method == EGPU_GCR || method == EGPU_BICGSTABL) return launch_ext(ctx, a, method, form, smem);
   }
-  if constexpr (sizeof(VT) == 4) {
-    if (a.sweeps_l > 0 && a.precond == EGPU_PREC_ILU0)
-      return offs ? launch_coop(ctx, bicgstab_kernel<float, TRI_TS, true, false, true>, a, nullptr, 0)
-                  : launch_coop(ctx, bicgstab_kernel<float, TRI_TS, false, false, true>, a, nullptr, 0);
-  }
-  if (cta) {
-    if (offs) return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, true, true>, a, nullptr, smem);
-    return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, false, true>, a, nullptr, smem);
-  }
-  if (offs) return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, true, false>, a, nullptr, smem);
-  return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, false, false>, a, nullptr, smem);
+  return launch_bicgstab(ctx, a, offs, form, smem);
 }
 
 // stored vectors of GCR (2 (m-1) directions) / BiCGStab(l) (r_0..r_l, u_0..u_l, shadow, x,
@@ -1177,6 +1165,7 @@ int solve_fp64(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_param
   set_sell(a, A, A->sell_vals.p, A->sell_c16.p != nullptr);
   a.ilu = A->ilu.p;
   a.dvals = dvals;
+  if (is_ilu(prm->precond) && (rc = range_pack(A, 0))) return rc;
   set_tri(a, A);
   a.precond = is_ilu(prm->precond) ? EGPU_PREC_ILU0 : prm->precond;  // ILUT applies like ILU(n)
   a.maxit = prm->max_iter;
@@ -1335,6 +1324,8 @@ int krylov_fp64_scaled(egpu_mat *A, const double *bs, double *xs, const egpu_par
   set_sell(a, A, A->sell_vals.p, A->sell_c16.p != nullptr);
   a.ilu = A->ilu.p;
   a.dvals = A->work.p + (size_t)11 * A->ldw;
+  int rc = is_ilu(prm->precond) ? range_pack(A, 0) : EGPU_OK;
+  if (rc) return rc;
   set_tri(a, A);
   a.precond = is_ilu(prm->precond) ? EGPU_PREC_ILU0 : prm->precond;  // ILUT applies like ILU(n)
   a.maxit = prm->max_iter;
@@ -1351,7 +1342,7 @@ int krylov_fp64_scaled(egpu_mat *A, const double *bs, double *xs, const egpu_par
   a.out_i = (int *)(ctx->sync.p + 8);
   a.out_d = (double *)(ctx->sync.p + 16);
   a.skip = nullptr;
-  int rc = run_krylov<double>(A, a, prm->method, A->sell_c16.p != nullptr);
+  rc = run_krylov<double>(A, a, prm->method, A->sell_c16.p != nullptr);
   if (rc) return rc;
   unsigned int h[64];
   EGPU_CUDA_TRY(ctx, cudaMemcpyAsync(h, ctx->sync.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1525,13 +1516,14 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
       a.ilu = A->ilu32.p;
       a.dvals = dv32;
       a.unit_diag = unit_diag ? 1 : 0;
+      if (ilu && !use_sweeps && (rc = range_pack(A, 1))) return rc;
       set_tri(a, A);
       if (use_sweeps) {
         a.sweeps_l = a.sweeps_u = sweeps;
         a.swr = A->sell_swr.p;
         a.isvals = A->ilu_sell32.p;
         a.idinv = A->ilu_dinv32.p;
-        a.tri_cta = 0;
+        a.tri_cta = a.rg_rows = 0;
       }
       a.precond = is_ilu(prm->precond) ? EGPU_PREC_ILU0 : prm->precond;  // ILUT applies like ILU(n)
       a.maxit = std::max(1, std::min(prm->inner_max_iter, prm->max_iter - r.iters));
@@ -1597,6 +1589,13 @@ __global__ void __launch_bounds__(EGPU_BLOCK, 2) k_lu_apply(KArgs<double> a, con
   (void)n;
 }
 
+// the same over the row ranges, one block per range
+template <int TRI>
+__global__ void __launch_bounds__(EGPU_KBLOCK, 1) k_lu_apply_range(KArgs<double> a, const double *v, double *u) {
+  range_init(a.rg_nt);
+  range_ilu<double, TRI>(a, a.w, u, [&](int i) { return v[i]; }, [](int, double) {});
+}
+
 // the same with the level-synchronous solves in one block (rhs gathered into slot order)
 __global__ void k_gather_slots(int n, const int *__restrict__ order, const double *__restrict__ v, double *slo) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) slo[s] = v[order[s]];
@@ -1625,11 +1624,12 @@ int lu_apply(egpu_mat *A, const double *v_dev, double *u_dev) {
   a.cols = A->cols.p;
   a.diag = A->diag.p;
   a.ilu = A->ilu.p;
+  int rc = range_pack(A, 0);
+  if (rc) return rc;
   set_tri(a, A);
   a.w = A->work.p;
   a.err = (int *)(ctx->sync.p + 1);
   a.tri_per_block = tri_per_block(A, TRI_TS, ctx->num_sms * 2, EGPU_BLOCK);
-  int rc;
   if (a.tri_cta) {
     const size_t smem = A->tri.cta_smem[0];
     if (smem > 48 * 1024)
@@ -1640,6 +1640,15 @@ int lu_apply(egpu_mat *A, const double *v_dev, double *u_dev) {
     k_lu_apply_block<<<1, EGPU_KBLOCK, smem, ctx->stream>>>(a, slo, yup, u_dev);
     ctx->launches += 2;
     rc = (int)cudaGetLastError();
+  } else if (a.rg_rows) {
+    const size_t smem = range_smem_bytes<double>(a.rg_rows, a.rg_ext, a.rg_stage);
+    const void *k = A->tri.rg_k == 10 ? (const void *)k_lu_apply_range<TRI_RANGE10>
+                                     : (const void *)k_lu_apply_range<TRI_RANGE7>;
+    if (smem > 48 * 1024)
+      EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    void *args[] = {&a, &v_dev, &u_dev};
+    rc = cudaLaunchCooperativeKernel(k, dim3((n + a.rg_rows - 1) / a.rg_rows),
+                                     dim3(EGPU_KBLOCK), args, smem, ctx->stream);
   } else {
     auto k = k_lu_apply<TRI_TS>;
     int bps = 0;

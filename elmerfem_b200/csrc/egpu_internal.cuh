@@ -149,6 +149,31 @@ struct CtaTriHost {
   DevBuf<int> map;
 };
 
+// One triangle of the row-range solve on the device (plan::RangeTriHost): offset[v] the byte
+// offsets of the level records (v = 0 FP64, 1 FP32), idx the shared-memory index of every padded
+// entry by global slot
+struct RangeTriDev {
+  DevBuf<int> lev_ptr, row, slot_lev, ext_ptr, ext;
+  DevBuf<int2> lev;
+  DevBuf<long long> offset[2];
+  long long bytes[2] = {0, 0};
+  DevBuf<uint16_t> slot, idx;
+  void view(const RangeTriDev &o) {
+    lev_ptr.view(o.lev_ptr);
+    row.view(o.row);
+    slot_lev.view(o.slot_lev);
+    ext_ptr.view(o.ext_ptr);
+    ext.view(o.ext);
+    lev.view(o.lev);
+    for (int v = 0; v < 2; ++v) {
+      offset[v].view(o.offset[v]);
+      bytes[v] = o.bytes[v];
+    }
+    slot.view(o.slot);
+    idx.view(o.idx);
+  }
+};
+
 struct TriSchedule {
   // rows in the order the sync-free solve processes them (ascending dependency level)
   DevBuf<int> lower_order, upper_order;
@@ -163,6 +188,11 @@ struct TriSchedule {
   // hold whole blocks (slots s*bs .. s*bs+bs-1: lower ascending, upper descending rows) and
   // the levels count blocks
   int bs = 1;
+  // row-range schedule (egpu_tri_range.h): rows per range (0: none), external cells, lanes and
+  // entries a lane, threads solving rows, bytes of a stage; rg_ok[v]: fits in FP64 (v = 0) / FP32 (v = 1)
+  int rg_rows = 0, rg_ext = 0, rg_g = 0, rg_k = 0, rg_nt = 0, rg_stage[2] = {0, 0};
+  bool rg_ok[2] = {false, false};
+  RangeTriDev rg_lo, rg_up;
   // level-synchronous single-block schedule; cta_ok[v] for FP64 (v = 0) / FP32 (v = 1)
   CtaTriHost cta_lo, cta_up;
   DevBuf<int> pos_lo, pos_up;        // solve slot of every row in the lower / upper order
@@ -211,6 +241,9 @@ struct egpu_mat {
   DevBuf<float> lo_vals32, up_vals32, up_dinv32;
   DevBuf<double> cta_lo_vals, cta_up_vals;        // the factors in the level-synchronous ELL layout
   DevBuf<float> cta_lo_vals32, cta_up_vals32;
+  // the level records of the row-range solves, packed when a solve first needs them (rg_packed[v])
+  DevBuf<unsigned char> rg_lo_rec[2], rg_up_rec[2];
+  bool rg_packed[2] = {false, false};
   DevBuf<int16_t> cols16;        // column offsets (col - row) when |col-row| < 32768
   DevBuf<int> ilu_done;          // factorisation completion flags
   // SELL-32 copy of the pattern (slice s = rows 32s..32s+31, entry (k, lane) at

@@ -18,10 +18,26 @@
 #pragma once
 
 #include "egpu_internal.cuh"
+#include "egpu_tri_range.h"
 
 namespace egpu {
 
 enum { SLOT_BB = 0, SLOT_RHO, SLOT_PQ, SLOT_RR, SLOT_SS, SLOT_TS, SLOT_TT, SLOT_RR2, NUM_SLOTS };
+
+// Forms of the ILU solves: sync-free (rows or node blocks; also the form of kernels without
+// ILU), level-synchronous in block 0, row ranges (7 or 10 entries a lane)
+enum TriForm { TRI_SYNCFREE = 0, TRI_CTA, TRI_RANGE7, TRI_RANGE10 };
+constexpr bool tri_range(int form) { return form == TRI_RANGE7 || form == TRI_RANGE10; }
+
+// One triangle of the row-range solve on the device: the level records of every range
+// (plan::range_records, with values), slot of every row, external rows
+struct RangeTri {
+  const int *lev_ptr;
+  const long long *offset;
+  const unsigned char *rec;
+  const uint16_t *slot;
+  const int *ext_ptr, *ext;
+};
 
 // One triangle of the level-synchronous solve (layout described at CtaTriHost)
 template <typename VT>
@@ -95,6 +111,11 @@ struct KArgs {
   long long ext_lds;
   const int *pos_lo, *pos_up;     // solve slot of each row, lower / upper order
   CtaTri<VT> clo, cup;
+  // row-range solves (range_ilu): rows per range (0: off), external cells, log2 lanes a row,
+  // threads that solve rows, bytes of a stage; the ILU structure's diagonal positions
+  int rg_rows, rg_ext, rg_lg, rg_nt, rg_stage;
+  RangeTri rlo, rup;
+  const int *idiag;
 };
 
 // row sum step: FP64 keeps CRS_MatrixVectorProd's rounding (s = s + a*x, two roundings, row
@@ -531,6 +552,341 @@ __device__ __forceinline__ void upper_solve_blk(const KArgs<VT> &a, const VT *y,
   }
 }
 
+// -------------------------------------------------------------------------------------
+// Row-range triangular solves (plan: egpu_tri_range.h).
+//
+// What bounds a solve is the chain of dependency levels.  Spread over all SMs, as above, every
+// level costs a store, an L2 round trip, a poll and a warp's sum (0.9 us; 1.7 us for a node
+// block).  Here a block owns a contiguous range of rows, whose values it keeps in shared memory
+// and solves level by level, one block barrier a level: G lanes a row, K entries a lane, all of
+// a level's rows at once, the entries staged by one bulk copy a level.  Only dependencies that cross a range boundary go through L2, and
+// those are off the chain: separate warps fetch them into shared memory as they are published.
+// (A warp per row polling shared memory was slower than no ranges at all: the polls of the
+// waiting warps take the issue slots and the shared-memory pipe from the warp on the chain.)
+//
+// Node blocks: the packed entries are premultiplied by the inverse of the block's own
+// triangle (k_range_pack), as are the right-hand sides, so the rows of a node depend on other
+// nodes only and the levels are those of the node graph.
+//
+// Shared memory: the level stages and their mbarriers, own values (rg_rows), external values
+// (rg_ext), a zero cell, right-hand sides (rg_rows).
+//
+// barrier among the first nt threads of the block (named barrier 1; nt a multiple of 32)
+__device__ __forceinline__ void cta_bar(int nt) { asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory"); }
+
+// mbarriers of the stages (copied; read), then the number of levels staged so far in this launch
+constexpr int RANGE_COUNT_AT = 16 * plan::RANGE_STAGES;
+constexpr int RANGE_FETCH = 8;   // warps fetching external values
+constexpr int RANGE_AHEAD = 16;  // levels prefetched into L2
+constexpr int RANGE_HEAD = 16 * ((RANGE_COUNT_AT + 4 + 15) / 16);
+// stage: bytes of the largest level record
+template <typename VT>
+__host__ __device__ constexpr size_t range_smem_bytes(int rows, int ext, int stage) {
+  return RANGE_HEAD + (size_t)plan::RANGE_STAGES * stage + sizeof(VT) * (size_t)(2 * rows + ext + 1);
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// one bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned), counted by bar
+__device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// every 64th round of a wait: true when it has to end (limit passed, or an error recorded)
+__device__ __forceinline__ bool range_wait_over(unsigned int spin, unsigned long long &t0, int *err) {
+  if (spin & 63u) return false;
+  if (*(volatile int *)err) return true;
+  const unsigned long long t = egpu_globaltimer();
+  if (t0 == 0) t0 = t;
+  if (t - t0 > egpu_wait_limit(err)) {
+    atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+    return true;
+  }
+  return false;
+}
+
+// does a value loaded from a cell hold the sentinel (its high word marks it: a NaN that arithmetic
+// never produces)
+__device__ __forceinline__ bool range_unset(double v) { return __double2hiint(v) == (int)(EGPU_SENTINEL64 >> 32); }
+__device__ __forceinline__ bool range_unset(float v) { return __float_as_uint(v) == EGPU_SENTINEL32; }
+
+template <typename VT>
+__device__ __forceinline__ VT range_lds(unsigned a) {
+  VT v;
+  if constexpr (sizeof(VT) == 8)
+    asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  else
+    asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+template <typename VT>
+__device__ __forceinline__ void range_sts(unsigned a, VT v) {
+  if constexpr (sizeof(VT) == 8)
+    asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+  else
+    asm volatile("st.volatile.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+// the scalars of a solve: shared-memory addresses (values, right-hand sides, stages), published
+// values, lanes a row (log2), threads that solve rows
+template <typename VT>
+struct RangeRun {
+  unsigned sx, srhs, stage, bar;
+  VT *x;
+  int *err;
+  int rows, stage_bytes, lg, nt;
+  unsigned first;  // levels staged before this triangle (stage and parity go on)
+};
+
+// named barriers 1 and 2 (nt a multiple of 32; the calling warp converged)
+__device__ __forceinline__ void range_sync(int id, int nt) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nt) : "memory"); }
+__device__ __forceinline__ void range_arrive(int id, int nt) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nt) : "memory"); }
+
+// One triangle of this block's range (not inlined: the Krylov kernels keep their registers, and
+// this loop its own).  Two sets of nt threads solve the levels in turn: while one set sums level
+// m, the other reads the entries of level m + 1 from its stage into registers, so between two
+// levels there is only a barrier, the loads of the values, the sum and a store (about 1,000
+// cycles a level with one set, which read its next entries in between).  The barrier that starts
+// level m: its set waits, the other arrives when level m - 1 is stored.
+// The next warp stages level records, RANGE_STAGES ahead; the rest fetch external values.
+// Returns the levels staged.
+template <typename VT, int K>
+__device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT> R) {
+  constexpr int S = plan::RANGE_STAGES;
+  const int b = blockIdx.x;
+  const int l0 = __ldg(T.lev_ptr + b), nl = __ldg(T.lev_ptr + b + 1) - l0;
+  const int nbar = 2 * R.nt;
+  if ((int)threadIdx.x < 2 * R.nt) {
+    const int set = (int)threadIdx.x >= R.nt ? 1 : 0, tid = (int)threadIdx.x - set * R.nt;
+    const int t = tid >> R.lg, G = 1 << R.lg;
+    VT v[K], r = 0;
+    unsigned xa[K];  // addresses of the entries' values
+    int row = -1;
+    unsigned dst = 0;
+    // the entries of level m, from its stage into registers
+    auto load = [&](int m) {
+      const unsigned q = R.first + m, st = q % S, bar = R.bar + 8 * st, ph = (q / S) & 1u;
+      row = -1;
+      bool here = mbar_try(bar, ph);
+      if (!here) {  // bounded; once an error is recorded, no level waits again or is solved
+        unsigned long long t0 = 0;
+        for (unsigned int spin = 64; !(here = mbar_try(bar, ph)); spin += 64)
+          if (range_wait_over(spin, t0, R.err)) break;
+      }
+      const unsigned rec = R.stage + st * (unsigned)R.stage_bytes;
+      int s0 = 0, w = 0;
+      if (here) asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(s0), "=r"(w) : "r"(rec));
+      if (t < w) {
+        const unsigned wg = (unsigned)w << R.lg;
+        const unsigned ia = rec + 16 + ((4u * w + 15) & ~15u);
+        const unsigned va = ia + ((2u * K * wg + 15) & ~15u);
+        asm volatile("ld.shared.s32 %0, [%1];" : "=r"(row) : "r"(rec + 16 + 4 * t));
+#pragma unroll
+        for (int k = 0; k < K; ++k) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(xa[k]) : "r"(ia + 2 * (k * wg + tid)));
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = range_lds<VT>(va + (unsigned)sizeof(VT) * (k * wg + tid));
+        r = 0;  // the row's right-hand side enters on its first lane
+        if ((tid & (G - 1)) == 0) r = range_lds<VT>(R.srhs + (unsigned)sizeof(VT) * (s0 + t));
+        dst = R.sx + (unsigned)sizeof(VT) * (s0 + t);
+#pragma unroll
+        for (int k = 0; k < K; ++k) xa[k] = R.sx + (unsigned)sizeof(VT) * xa[k];
+      }
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(bar + 8 * S);  // this warp has read the stage
+    };
+    if (set < nl) load(set);
+    __syncwarp();
+    if (set == 1 && nl > 0) range_arrive(1, nbar);
+    for (int m = set; m < nl; m += 2) {
+      range_sync(1 + (m & 1), nbar);
+      VT acc = 0;
+      if (row >= 0) {
+        VT xv[K];
+        bool unset = false;
+#pragma unroll
+        for (int k = 0; k < K; ++k) xv[k] = range_lds<VT>(xa[k]);
+#pragma unroll
+        for (int k = 0; k < K; ++k) unset |= range_unset(xv[k]);
+        if (unset) {  // external values that have not arrived
+          unsigned long long t0 = 0;
+          for (unsigned int spin = 1; unset; ++spin) {
+            unset = false;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+              xv[k] = range_lds<VT>(xa[k]);
+              unset |= range_unset(xv[k]);
+            }
+            if (unset && range_wait_over(spin, t0, R.err)) break;
+          }
+        }
+        // four chains: the FP64 units' latency (about 60 cycles an operation) is the level's time
+        VT p[4] = {r, VT(0), VT(0), VT(0)};
+#pragma unroll
+        for (int k = 0; k < K; ++k) p[k & 3] -= v[k] * xv[k];
+        acc = (p[0] + p[1]) + (p[2] + p[3]);
+      }
+      __syncwarp();
+      for (int off = G >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      const VT z = acc;
+      if (row >= 0 && (tid & (G - 1)) == 0) range_sts<VT>(dst, z);
+      __syncwarp();
+      if (m + 1 < nl) range_arrive(1 + ((m + 1) & 1), nbar);
+      if (row >= 0 && (tid & (G - 1)) == 0) Sentinel<VT>::publish(R.x + row, z);
+      if (m + 2 < nl) load(m + 2);
+      __syncwarp();
+    }
+  } else if ((int)threadIdx.x < nbar + 32) {
+    // One thread issues.  It reuses a stage when all warps of the set have read it and the copy
+    // before is complete (it is, except after an error, when the solving threads stop waiting),
+    // so at most RANGE_STAGES are in flight, and after an error it sees those end too.
+    if ((int)threadIdx.x == nbar) {
+      auto wait = [&](unsigned bar, unsigned ph) {
+        if (mbar_try(bar, ph)) return true;
+        const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(R.err);
+        while (!mbar_try(bar, ph))
+          if (egpu_globaltimer() - t0 > lim) {
+            atomicExch(R.err, (int)EGPU_ERR_TIMEOUT);
+            return false;
+          }
+        return true;
+      };
+      auto bar = [&](unsigned q) { return R.bar + 8 * (q % S); };
+      auto phase = [&](unsigned q) { return (q / S) & 1u; };
+      int l = 0;
+      long long o0 = __ldg(T.offset + l0);
+      for (; l < nl; ++l) {
+        const unsigned q = R.first + l;
+        const long long o1 = __ldg(T.offset + l0 + l + 1);
+        if (q >= S && (!wait(bar(q) + 8 * S, phase(q - S)) || !wait(bar(q), phase(q - S)))) break;
+        bulk_load(R.stage + (q % S) * (unsigned)R.stage_bytes, T.rec + o0, (unsigned)(o1 - o0), bar(q));
+        o0 = o1;
+        // the level RANGE_AHEAD later into L2: the stages alone cover an L2 hit, not HBM
+        if (l + RANGE_AHEAD < nl) {
+          const long long p0 = __ldg(T.offset + l0 + l + RANGE_AHEAD), p1 = __ldg(T.offset + l0 + l + RANGE_AHEAD + 1);
+          prefetch_l2_bulk(T.rec + p0, (unsigned)(p1 - p0));
+        }
+      }
+      if (*(volatile int *)R.err)
+        for (int h = max(0, l - S); h < l; ++h) wait(bar(R.first + h), phase(R.first + h));
+    }
+  } else {
+    // External values, in the order of their first use, 32 a warp at a time, by at most
+    // RANGE_FETCH warps (twenty polling warps an SM took a third of the L2's bandwidth)
+    const int f = ((int)threadIdx.x - nbar - 32) >> 5, nf = min(RANGE_FETCH, ((int)blockDim.x - nbar - 32) >> 5);
+    const int e0 = __ldg(T.ext_ptr + b), e1 = __ldg(T.ext_ptr + b + 1), lane = threadIdx.x & 31;
+    int e = e0 + 32 * f + lane;
+    int next = f < nf && e < e1 ? __ldg(T.ext + e) : -1;
+    for (int q = e0 + 32 * f; f < nf && q < e1; q += 32 * nf, e += 32 * nf) {
+      const VT *p = next >= 0 ? R.x + next : nullptr;
+      next = e + 32 * nf < e1 ? __ldg(T.ext + e + 32 * nf) : -1;
+      bool pend = p != nullptr;
+      unsigned long long t0 = 0;
+      for (unsigned int spin = 1; __any_sync(0xffffffffu, pend); ++spin) {
+        if (pend) {
+          const VT v = Sentinel<VT>::peek(p);
+          if (!Sentinel<VT>::is(v)) {
+            range_sts<VT>(R.sx + (unsigned)sizeof(VT) * (R.rows + e - e0), v);
+            pend = false;
+          } else if (range_wait_over(spin, t0, R.err)) {
+            pend = false;
+          }
+        }
+      }
+    }
+  }
+  return nl;
+}
+
+// Once per launch, by all threads of every block, before the first range_ilu: the stages'
+// mbarriers (one object for the whole launch: their phases go on from solve to solve)
+__device__ __forceinline__ void range_init(int nt) {
+  extern __shared__ __align__(16) unsigned char egpu_dsm[];
+  if (threadIdx.x < 2 * plan::RANGE_STAGES)
+    mbar_init(smem_u32(egpu_dsm) + 8 * threadIdx.x, threadIdx.x < plan::RANGE_STAGES ? 1u : (unsigned)nt / 32);
+  if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned *>(egpu_dsm + RANGE_COUNT_AT) = 0u;
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+}
+
+// z = (LU)^-1 rhs in the row-range form, called by all threads of every block: rhs(i) once for
+// each of the block's own rows, out(i, z_i) for them at the end.  y and z (published values) hold
+// the sentinel on entry.
+template <typename VT, int TRI, typename RHS, typename OUT>
+__device__ __forceinline__ void range_ilu(const KArgs<VT> &a, VT *y, VT *z, RHS &&rhs, OUT &&out) {
+  constexpr int K = TRI == TRI_RANGE10 ? 10 : 7;
+  extern __shared__ __align__(16) unsigned char egpu_dsm[];
+  unsigned char *stage = egpu_dsm + RANGE_HEAD;
+  VT *sx = reinterpret_cast<VT *>(stage + (size_t)plan::RANGE_STAGES * a.rg_stage);
+  VT *srhs = sx + a.rg_rows + a.rg_ext + 1;
+  volatile unsigned *count = reinterpret_cast<volatile unsigned *>(egpu_dsm + RANGE_COUNT_AT);
+  const int base = blockIdx.x * a.rg_rows, cnt = min(a.rg_rows, a.n - base), bs = a.tri_bs;
+  __syncthreads();  // the buffer's previous use is over
+  for (int i = threadIdx.x; i <= a.rg_ext; i += blockDim.x) sx[a.rg_rows + i] = i < a.rg_ext ? Sentinel<VT>::value() : VT(0);
+  // right-hand sides times the inverse of the node block's unit lower triangle
+  for (int i = threadIdx.x * bs; i < cnt; i += blockDim.x * bs) {
+    VT t[TRI_BS_MAX];
+#pragma unroll
+    for (int k = 0; k < TRI_BS_MAX; ++k)
+      if (k < bs) {
+        const int r = base + i + k;
+        VT v = rhs(r);
+        if (k > 0) {
+          const int dg = __ldg(a.idiag + r);
+#pragma unroll
+          for (int j = 0; j < k; ++j) v -= __ldg(a.ilu + dg - k + j) * t[j];
+        }
+        t[k] = v;
+        srhs[__ldg(a.rlo.slot + r)] = v;
+      }
+  }
+  __syncthreads();
+  RangeRun<VT> run{smem_u32(sx), smem_u32(srhs), smem_u32(stage), smem_u32(egpu_dsm), y,       a.err,
+                   a.rg_rows,    a.rg_stage,     a.rg_lg,         a.rg_nt,            *count};
+  if (cnt > 0) run.first += (unsigned)range_triangle<VT, K>(a.rlo, run);
+  __syncthreads();
+  for (int i = threadIdx.x; i < a.rg_ext; i += blockDim.x) sx[a.rg_rows + i] = Sentinel<VT>::value();
+  // y times the inverse of the node block's upper triangle (inverted diagonal included)
+  for (int i = threadIdx.x * bs; i < cnt; i += blockDim.x * bs) {
+    VT t[TRI_BS_MAX];
+#pragma unroll
+    for (int q = 0; q < TRI_BS_MAX; ++q) {
+      const int k = TRI_BS_MAX - 1 - q;  // row of the block, last first
+      if (k < bs) {
+        const int r = base + i + k, dg = __ldg(a.idiag + r);
+        VT v = sx[__ldg(a.rlo.slot + r)];
+#pragma unroll
+        for (int j = k + 1; j < TRI_BS_MAX; ++j)
+          if (j < bs) v -= __ldg(a.ilu + dg + j - k) * t[j];
+        t[k] = __ldg(a.ilu + dg) * v;
+        srhs[__ldg(a.rup.slot + r)] = t[k];
+      }
+    }
+  }
+  __syncthreads();
+  run.x = z;
+  if (cnt > 0) run.first += (unsigned)range_triangle<VT, K>(a.rup, run);
+  __syncthreads();
+  if (threadIdx.x == 0) *count = run.first;
+  for (int i = threadIdx.x; i < cnt; i += blockDim.x) out(base + i, sx[__ldg(a.rup.slot + base + i)]);
+}
+
 // lower: y_i = rhs_i - sum_{j<i} L_ij y_j (CRS_LUSolve forward, CRSMatrix.src:3346-3352).
 // One warp per slot; the next slot's row and entries are fetched while this slot waits.
 template <typename VT, int TS, typename RHS>
@@ -660,8 +1016,6 @@ struct CtaPos {
 
 __device__ __forceinline__ int cta_wrap(int i, int n) { return i >= n ? i - n : i; }
 
-// barrier among the first nt threads of the block (named barrier 1; nt a multiple of 32)
-__device__ __forceinline__ void cta_bar(int nt) { asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory"); }
 
 // issue the copies of level lv (window positions p) into the staging windows (threads
 // 0..nt-1)
@@ -886,15 +1240,13 @@ __device__ __forceinline__ bool sweep_apply(const KArgs<float> &a, const float *
 }
 
 // =====================================================================================
-// Every persistent Krylov kernel is instantiated twice: CTA = true carries the
-// level-synchronous triangular solves of block 0 (chosen per matrix when its levels are
-// narrow), CTA = false leaves them out, so the kernels of the other schedules keep the
-// registers those solves would take.
+// Every persistent Krylov kernel is instantiated per form of the ILU solves (TriForm, chosen
+// per matrix), so that no form pays the registers of another.
 //
 // CG  (huti_dcgsolv, hutiter/src/huti_cg_D.F90:84-257)
 //
 // w layout: R Z P Q Y(ILU lower result)
-template <typename VT, int LPR, bool OFFS, bool CTA>
+template <typename VT, int LPR, bool OFFS, int TRI>
 __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
   if (a.skip && (*a.skip & 2u)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -907,6 +1259,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
   __shared__ double sm[32 * 4];
   unsigned int epoch = 0;
   const int n = a.n;
+  if constexpr (tri_range(TRI)) range_init(a.rg_nt);
 
   const int nb = gridDim.x;
   const bool ilu = a.precond == EGPU_PREC_ILU0;
@@ -915,7 +1268,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
   VT *X = a.x, *R = a.w, *Z = zr ? a.w : a.w + a.ldw, *P = a.w + 2 * a.ldw, *Q = a.w + 3 * a.ldw,
      *Y = a.w + 4 * a.ldw;
   const VT *B = a.b;
-  const bool cta = CTA && ilu && a.tri_cta;  // block 0 runs the ILU0 solves level-synchronously
+  const bool cta = TRI == TRI_CTA && ilu && a.tri_cta;  // block 0 runs the ILU0 solves level-synchronously
   const VT SENT = Sentinel<VT>::value();
   // level-synchronous mode: R in lower / upper slot order, y in upper slot order
   VT *SLO = a.w + 4 * a.ldw, *YUP = a.w + 5 * a.ldw, *AUX = a.w + 6 * a.ldw;
@@ -972,8 +1325,12 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
       if (blockIdx.x == 0)
         cta_ilu(a, SLO, YUP, AUX, Z, [&](int, VT zi, VT ri) { acc[0] += (double)ri * (double)zi; });
     } else if (ilu) {
-      lower_solve<VT, LPR>(a, Y, [&](int i) { return R[i]; });
-      upper_solve<VT, LPR>(a, Y, Z, [&](int i, VT zi) { acc[0] += (double)R[i] * (double)zi; });
+      if constexpr (tri_range(TRI)) {
+        range_ilu<VT, TRI>(a, Y, Z, [&](int i) { return R[i]; }, [&](int i, VT zi) { acc[0] += (double)R[i] * (double)zi; });
+      } else {
+        lower_solve<VT, LPR>(a, Y, [&](int i) { return R[i]; });
+        upper_solve<VT, LPR>(a, Y, Z, [&](int i, VT zi) { acc[0] += (double)R[i] * (double)zi; });
+      }
     } else {
       const bool jac = a.precond == EGPU_PREC_DIAGONAL && !zr;
       vec_loop<VT>(n, [&](int i, auto w) {
@@ -1092,14 +1449,24 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
         store_partials(a, SLOT_RHO, rh[0]);
       } else {
         if (ilu) {
-          lower_solve<VT, LPR>(a, Y, [&](int i) { return R[i] - alpha * Q[i]; });
-          upper_solve<VT, LPR>(a, Y, Z, [&](int i, VT zi) {
-            const VT r = R[i] - alpha * Q[i];
-            R[i] = r;
-            X[i] = X[i] + alpha * P[i];
-            acc[0] += (double)r * (double)zi;
-            acc[1] += (double)r * (double)r;
-          });
+          if constexpr (tri_range(TRI)) {
+            range_ilu<VT, TRI>(a, Y, Z, [&](int i) {
+              const VT r = R[i] - alpha * Q[i];
+              R[i] = r;
+              X[i] = X[i] + alpha * P[i];
+              acc[1] += (double)r * (double)r;
+              return r;
+            }, [&](int i, VT zi) { acc[0] += (double)R[i] * (double)zi; });
+          } else {
+            lower_solve<VT, LPR>(a, Y, [&](int i) { return R[i] - alpha * Q[i]; });
+            upper_solve<VT, LPR>(a, Y, Z, [&](int i, VT zi) {
+              const VT r = R[i] - alpha * Q[i];
+              R[i] = r;
+              X[i] = X[i] + alpha * P[i];
+              acc[0] += (double)r * (double)zi;
+              acc[1] += (double)r * (double)r;
+            });
+          }
         } else {
           const bool jac = a.precond == EGPU_PREC_DIAGONAL && !zr;
           vec_loop<VT>(n, [&](int i, auto w) {
@@ -1149,7 +1516,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
 // BiCGStab  (huti_dbicgstabsolv, hutiter/src/huti_bicgstab_D.F90:96-284)
 //
 // w layout: R RTLD P V T S T1V T2V Y1 Y2
-template <typename VT, int LPR, bool OFFS, bool CTA, bool SW = false>
+template <typename VT, int LPR, bool OFFS, int TRI, bool SW = false>
 __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
   if (a.skip && (*a.skip & 2u)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1162,6 +1529,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
   __shared__ double sm[32 * 4];
   unsigned int epoch = 0;
   const int n = a.n;
+  if constexpr (tri_range(TRI)) range_init(a.rg_nt);
 
   const int nb = gridDim.x;
   VT *X = a.x;
@@ -1171,7 +1539,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
   const VT *B = a.b;
   const bool ilu = a.precond == EGPU_PREC_ILU0;
   const bool jac = a.precond == EGPU_PREC_DIAGONAL;
-  const bool cta = CTA && ilu && a.tri_cta;  // block 0 runs the ILU0 solves level-synchronously
+  const bool cta = TRI == TRI_CTA && ilu && a.tri_cta;  // block 0 runs the ILU0 solves level-synchronously
   // FP32 inner solves: ILU0 by Jacobi sweeps (Y1, Y2 and work vector 12 as scratch)
   constexpr bool sw = SW && sizeof(VT) == 4;
   const bool syncfree = ilu && !cta && !sw;
@@ -1293,12 +1661,17 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
         if (!grid_barrier(a.bar, a.err, epoch)) return;
         if (blockIdx.x == 0) cta_ilu(a, SLO, YUP, (const VT *)nullptr, T1, [](int, VT, VT) {});
       } else if (ilu) {
-        lower_solve<VT, LPR>(a, Y1, [&](int i) {
+        auto rhs = [&](int i) {
           const VT p = R[i] + beta * (P[i] - om * V[i]);
           P[i] = p;
           return p;
-        });
-        upper_solve<VT, LPR>(a, Y1, T1, [&](int, VT) {});
+        };
+        if constexpr (tri_range(TRI)) {
+          range_ilu<VT, TRI>(a, Y1, T1, rhs, [](int, VT) {});
+        } else {
+          lower_solve<VT, LPR>(a, Y1, rhs);
+          upper_solve<VT, LPR>(a, Y1, T1, [&](int, VT) {});
+        }
       } else {
         vec_loop<VT>(n, [&](int i, auto w) {
           constexpr int W = decltype(w)::value;
@@ -1392,13 +1765,18 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
         if (blockIdx.x == 0) cta_ilu(a, SLO, YUP, (const VT *)nullptr, T2, [](int, VT, VT) {});
       } else {
         if (ilu) {
-          lower_solve<VT, LPR>(a, Y2, [&](int i) {
+          auto rhs = [&](int i) {
             const VT s = row_msub(R[i], al, V[i]);
             S[i] = s;
             acc[0] += (double)s * (double)s;
             return s;
-          });
-          upper_solve<VT, LPR>(a, Y2, T2, [&](int, VT) {});
+          };
+          if constexpr (tri_range(TRI)) {
+            range_ilu<VT, TRI>(a, Y2, T2, rhs, [](int, VT) {});
+          } else {
+            lower_solve<VT, LPR>(a, Y2, rhs);
+            upper_solve<VT, LPR>(a, Y2, T2, [&](int, VT) {});
+          }
         } else {
           vec_loop<VT>(n, [&](int i, auto w) {
             constexpr int W = decltype(w)::value;
@@ -1516,7 +1894,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
 //
 // w layout: R T1 T2 Y(ILU lower result) SLO YUP(level-synchronous slot order)
 // stored directions: S_i = ext + i * ext_lds, V_i = ext + (m - 1 + i) * ext_lds, i < m - 1
-template <int LPR, bool CTA>
+template <int LPR, int TRI>
 __global__ void __launch_bounds__(EGPU_KBLOCK, 1) gcr_kernel(KArgs<double> a) {
   using VT = double;
   struct {
@@ -1535,11 +1913,12 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) gcr_kernel(KArgs<double> a) {
   __shared__ double sm[32 * 4];
   unsigned int epoch = 0;
   const int n = a.n, nb = gridDim.x;
+  if constexpr (tri_range(TRI)) range_init(a.rg_nt);
   VT *X = a.x, *R = a.w, *T1 = a.w + a.ldw, *T2 = a.w + 2 * a.ldw, *Y = a.w + 3 * a.ldw,
      *SLO = a.w + 4 * a.ldw, *YUP = a.w + 5 * a.ldw;
   const VT *B = a.b;
   const bool ilu = a.precond == EGPU_PREC_ILU0, jac = a.precond == EGPU_PREC_DIAGONAL;
-  const bool cta = CTA && ilu && a.tri_cta;
+  const bool cta = TRI == TRI_CTA && ilu && a.tri_cta;
   const VT SENT = Sentinel<VT>::value();
   // per row after r changed: prepare the next M^-1 (sentinels, or r in slot order)
   auto prep = [&](int i, VT r) {
@@ -1590,8 +1969,12 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) gcr_kernel(KArgs<double> a) {
     if (cta) {
       if (blockIdx.x == 0) cta_ilu(a, SLO, YUP, (const VT *)nullptr, T1, [](int, VT, VT) {});
     } else if (ilu) {
-      lower_solve<VT, 32>(a, Y, [&](int i) { return R[i]; });
-      upper_solve<VT, 32>(a, Y, T1, [&](int, VT) {});
+      if constexpr (tri_range(TRI)) {
+        range_ilu<VT, TRI>(a, Y, T1, [&](int i) { return R[i]; }, [](int, VT) {});
+      } else {
+        lower_solve<VT, 32>(a, Y, [&](int i) { return R[i]; });
+        upper_solve<VT, 32>(a, Y, T1, [&](int, VT) {});
+      }
     } else {
       vec_loop<VT>(n, [&](int i, auto w) {
         constexpr int W = decltype(w)::value;
@@ -1749,7 +2132,7 @@ __device__ inline void bl_lu_solve(int m, const double *a, int lda, const int *p
 
 constexpr int BL_MAXL = 8;
 
-template <int LPR, bool CTA>
+template <int LPR, int TRI>
 __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstabl_kernel(KArgs<double> a) {
   using VT = double;
   if (a.skip && (*a.skip & 2u)) {
@@ -1764,6 +2147,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstabl_kernel(KArgs<double>
   __shared__ double Zs[(BL_MAXL + 1) * (BL_MAXL + 1)], y0s[BL_MAXL + 1];
   unsigned int epoch = 0;
   const int n = a.n, nb = gridDim.x, l = a.ext_m, L1 = l + 1;
+  if constexpr (tri_range(TRI)) range_init(a.rg_nt);
   const long long ld = a.ext_lds;
   auto rv = [&](int j) { return a.ext + (long long)j * ld; };
   auto uv = [&](int j) { return a.ext + (long long)(L1 + j) * ld; };
@@ -1771,7 +2155,7 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstabl_kernel(KArgs<double>
   VT *X = a.x, *Y = a.w + 3 * a.ldw, *SLO = a.w + 4 * a.ldw, *YUP = a.w + 5 * a.ldw;
   const VT *B = a.b;
   const bool ilu = a.precond == EGPU_PREC_ILU0, jac = a.precond == EGPU_PREC_DIAGONAL;
-  const bool cta = CTA && ilu && a.tri_cta;
+  const bool cta = TRI == TRI_CTA && ilu && a.tri_cta;
   const VT SENT = Sentinel<VT>::value();
   double *gram = a.partials + 16 * nb;  // (l+1)(l+2)/2 slots of nb partials
   // dst = M^-1 src (pcondlsubr); ends after a grid barrier
@@ -1793,8 +2177,12 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstabl_kernel(KArgs<double>
       if (cta) {
         if (blockIdx.x == 0) cta_ilu(a, SLO, YUP, (const VT *)nullptr, dst, [](int, VT, VT) {});
       } else {
-        lower_solve<VT, 32>(a, Y, [&](int i) { return src[i]; });
-        upper_solve<VT, 32>(a, Y, dst, [&](int, VT) {});
+        if constexpr (tri_range(TRI)) {
+          range_ilu<VT, TRI>(a, Y, dst, [&](int i) { return src[i]; }, [](int, VT) {});
+        } else {
+          lower_solve<VT, 32>(a, Y, [&](int i) { return src[i]; });
+          upper_solve<VT, 32>(a, Y, dst, [&](int, VT) {});
+        }
       }
     } else {
       vec_loop<VT>(n, [&](int i, auto w) {

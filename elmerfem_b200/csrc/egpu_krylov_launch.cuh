@@ -1,0 +1,46 @@
+// egpu_krylov_launch.cuh -- launches of the persistent Krylov kernels.  Each method's kernels
+// are instantiated in a translation unit of their own (egpu_kcg.cu, egpu_kbicgstab.cu,
+// egpu_kext.cu).
+#pragma once
+
+#include <algorithm>
+
+#include "egpu_krylov.cuh"
+
+namespace egpu {
+
+// One warp per row in the sync-free triangular solves: rows that depend on each other
+// never share a warp, so no lane spins while a diverged lane of its own warp has to
+// produce the value it waits for.
+constexpr int TRI_TS = 32;
+
+// occupancy-sized cooperative launch
+template <typename K, typename Args>
+int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, size_t smem = 0) {
+  int bps = 0;
+  if (smem > 48 * 1024)
+    EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)smem));
+  EGPU_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, EGPU_KBLOCK, smem));
+  if (bps < 1) {
+    egpu_set_error(ctx, "persistent kernel does not fit on an SM");
+    return EGPU_ERR_CUDA;
+  }
+  bps = std::min(bps, 2048 / EGPU_KBLOCK);
+  int grid = ctx->num_sms * bps;
+  if (grid_out) *grid_out = grid;
+  void *kargs[] = {&args};
+  EGPU_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(EGPU_KBLOCK),
+                                                 kargs, smem, ctx->stream));
+  ctx->launches++;
+  return EGPU_OK;
+}
+
+// offs: 16-bit column offsets; form: a TriForm; smem: dynamic shared memory per block
+int launch_cg(egpu_ctx *ctx, KArgs<double> &a, bool offs, int form, size_t smem);
+int launch_cg(egpu_ctx *ctx, KArgs<float> &a, bool offs, int form, size_t smem);
+int launch_bicgstab(egpu_ctx *ctx, KArgs<double> &a, bool offs, int form, size_t smem);
+int launch_bicgstab(egpu_ctx *ctx, KArgs<float> &a, bool offs, int form, size_t smem);  // sweeps: a.sweeps_l > 0
+int launch_ext(egpu_ctx *ctx, KArgs<double> &a, int method, int form, size_t smem);     // GCR, BiCGStab(l)
+
+}  // namespace egpu

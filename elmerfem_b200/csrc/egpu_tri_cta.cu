@@ -12,8 +12,10 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "egpu_krylov.cuh"
 #include "egpu_solve.h"
 #include "egpu_tri_plan.h"
+#include "egpu_tri_range.h"
 
 namespace egpu {
 
@@ -25,11 +27,13 @@ constexpr size_t CTA_SMEM_MAX = 200 * 1024;
 
 int tri_mode_env() {
   // EGPU_TRI_MODE: "syncfree" never uses the single-block solve, "block" uses it whenever
-  // the schedule fits, anything else chooses by the cost estimate
+  // the schedule fits, "range" uses the row-range solve whenever it fits, anything else
+  // chooses by the cost estimates
   const char *m = std::getenv("EGPU_TRI_MODE");
   if (!m) return 0;
   if (!std::strcmp(m, "syncfree")) return 1;
   if (!std::strcmp(m, "block")) return 2;
+  if (!std::strcmp(m, "range")) return 3;
   return 0;
 }
 
@@ -171,6 +175,250 @@ bool cta_use(const egpu_mat *A, int v) {
   if (mode == 1) return false;
   if (mode == 2) return true;
   return est_block(S.cta_lo.nlev, S.cta_up.nlev, A->n) < est_syncfree(S.cta_lo.nlev, S.cta_up.nlev, A->n);
+}
+
+// Row-range solves when their modelled time (cycles at the 1.9 GHz the cards run at, plus the
+// passes over the right-hand side) beats the estimates of the other schedules.  The number of
+// ranges is the best of a few: fewer mean fewer hand-overs through L2, more mean narrower
+// levels and less shared memory.  Own values, external values and right-hand sides of a range
+// have to fit in shared memory (RANGE_SMEM of the 227 KB), in FP64 if any number of ranges
+// allows it, else in FP32 only.
+// shared-memory index of every padded entry (by global slot): the own row's slot, an external
+// row's cell, or the zero cell
+template <bool LOWER>
+__global__ void k_range_index(int n, int bs, int per, int gk, int zero, const int *__restrict__ row,
+                              const uint16_t *__restrict__ slot, const int *__restrict__ ext_ptr,
+                              const int2 *__restrict__ sorted, const int *__restrict__ rows,
+                              const int *__restrict__ cols, const int *__restrict__ diag, uint16_t *__restrict__ idx) {
+  const long long tot = (long long)n * gk;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
+    const int gs = (int)(q / gk), e = (int)(q % gk), c = gs / per, r0 = c * per;
+    const int r = row[gs], rb = r / bs * bs, e_lo = diag[rb] - rows[rb], len = rows[rb + 1] - rows[rb];
+    const int beg = rows[r] + (LOWER ? 0 : e_lo + bs), ne = LOWER ? e_lo : len - e_lo - bs;
+    int x = zero;
+    if (e < ne) {
+      const int d = cols[beg + e];
+      if (d >= r0 && d < min(n, r0 + per)) {
+        x = slot[d];
+      } else {
+        int lo = ext_ptr[c], hi = ext_ptr[c + 1] - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (sorted[mid].x < d)
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
+        x = per + sorted[lo].y;
+      }
+    }
+    idx[q] = (uint16_t)x;
+  }
+}
+
+constexpr size_t RANGE_SMEM = 216 * 1024;
+constexpr double RANGE_PASSES = 8e-6;
+
+int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vector<int> &cols,
+                         const std::vector<int> &diag, const std::vector<int> &lev_lo,
+                         const std::vector<int> &lev_up) {
+  egpu_ctx *ctx = A->ctx;
+  TriSchedule &S = A->tri;
+  const int n = A->n, bs = S.bs, mode = tri_mode_env();
+  S.rg_rows = 0;
+  S.rg_ok[0] = S.rg_ok[1] = false;
+  A->rg_packed[0] = A->rg_packed[1] = false;
+  if (mode == 1 || mode == 2) return EGPU_OK;
+  int most = 0;
+  for (int r = 0; r < n; r += bs) {
+    int beg, ne;
+    plan::range_entries(bs, true, rows, diag, r, beg, ne);
+    most = std::max(most, ne);
+    plan::range_entries(bs, false, rows, diag, r, beg, ne);
+    most = std::max(most, ne);
+  }
+  const plan::RangeShape sh = plan::range_shape(most);
+  if (sh.g == 0) return EGPU_OK;
+  const int forced = std::getenv("EGPU_TRI_RANGES") ? std::atoi(std::getenv("EGPU_TRI_RANGES")) : 0;
+  plan::RangeTriHost lo, up, best_lo, best_up;
+  double best = 0.0;
+  int best_per = 0, best_fit = 2;
+  for (int div : {1, 2, 3, 4, 6, 9, 12, 18, 37, 148}) {
+    if (forced && div > 1) break;
+    const int nr = std::max(1, std::min(ctx->num_sms, forced ? forced : ctx->num_sms / div));
+    const int per = ((n + nr - 1) / nr + bs - 1) / bs * bs;
+    if (range_smem_bytes<float>(per, 0, 0) > RANGE_SMEM || per > 32000) break;
+    if (!plan::range_triangle(n, bs, per, sh, true, rows, cols, diag, lev_lo, lo) ||
+        !plan::range_triangle(n, bs, per, sh, false, rows, cols, diag, lev_up, up))
+      continue;
+    const int ext = std::max(lo.max_ext, up.max_ext), maxr = std::max(lo.max_rows, up.max_rows);
+    auto bytes = [&](int vsize) { return plan::range_record(maxr, sh.g * sh.k, vsize); };
+    const int fit = range_smem_bytes<double>(per, ext, bytes(8)) <= RANGE_SMEM  ? 0
+                    : range_smem_bytes<float>(per, ext, bytes(4)) <= RANGE_SMEM ? 1
+                                                                                : 2;
+    if (fit == 2 || fit > best_fit) continue;
+    const double t = (plan::range_cycles(n, bs, per, sh, ext, true, rows, cols, diag, lev_lo) +
+                      plan::range_cycles(n, bs, per, sh, ext, false, rows, cols, diag, lev_up)) / 1.9e9 + RANGE_PASSES;
+    if (best_per == 0 || fit < best_fit || t < best) {
+      best = t;
+      best_per = per;
+      best_fit = fit;
+      std::swap(lo, best_lo);
+      std::swap(up, best_up);
+    }
+  }
+  if (best_per == 0) return EGPU_OK;
+  // measured per application: sync-free 0.8 us a level + 0.24 ns a row, node blocks 1.25 us +
+  // 0.4 ns (hex 32^3 372 us, 96^3 1,335 us; elasticity 24^3 440 us, 64^3 1,430 us), where the
+  // row ranges take 185, 1,090, 230 and 1,600 us
+  const double levels = S.lower_levels + S.upper_levels;
+  double other = bs > 1 ? 1.25e-6 * levels + 0.4e-9 * n : 0.8e-6 * levels + 0.24e-9 * n;
+  if (S.cta_ok[best_fit]) other = std::min(other, est_block(S.cta_lo.nlev, S.cta_up.nlev, n));
+  if (mode != 3 && 1.15 * best >= other) return EGPU_OK;  // the model's scatter
+  const int ext = std::max(best_lo.max_ext, best_up.max_ext);
+  const int gk = sh.g * sh.k;
+  auto upload = [&](const plan::RangeTriHost &T, bool lower, RangeTriDev &D) -> int {
+    static_assert(sizeof(plan::RangeLevel) == sizeof(int2), "levels are read as int2");
+    auto put = [&](auto &dst, const auto &src) -> int {
+      EGPU_CUDA_TRY(ctx, dst.alloc(std::max<size_t>(1, src.size())));
+      if (!src.empty())
+        EGPU_CUDA_TRY(ctx, cudaMemcpy(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
+      return EGPU_OK;
+    };
+    int rc = put(D.lev_ptr, T.lev_ptr);
+    if (!rc) rc = put(D.lev, T.lev);
+    if (!rc) rc = put(D.slot_lev, T.slot_lev);
+    if (!rc) rc = put(D.row, T.row);
+    if (!rc) rc = put(D.slot, T.slot);
+    if (!rc) rc = put(D.ext_ptr, T.ext_ptr);
+    if (!rc) rc = put(D.ext, T.ext);
+    for (int v = 0; v < 2 && !rc; ++v) {
+      std::vector<long long> off(T.lev.size() + 1, 0);
+      for (size_t l = 0; l < T.lev.size(); ++l)
+        off[l + 1] = off[l] + plan::range_record(T.lev[l].rows, gk, v == 0 ? 8 : 4);
+      D.bytes[v] = off.back();
+      rc = put(D.offset[v], off);
+    }
+    if (rc) return rc;
+    // shared-memory indices, on the device: external rows through a sorted copy of each list
+    std::vector<int2> sorted(std::max<size_t>(1, T.ext.size()));
+    for (size_t c = 0; c + 1 < T.ext_ptr.size(); ++c) {
+      for (int q = T.ext_ptr[c]; q < T.ext_ptr[c + 1]; ++q) sorted[q] = make_int2(T.ext[q], q - T.ext_ptr[c]);
+      std::sort(sorted.begin() + T.ext_ptr[c], sorted.begin() + T.ext_ptr[c + 1],
+                [](int2 x, int2 y) { return x.x < y.x; });
+    }
+    DevBuf<int2> ds;
+    rc = put(ds, sorted);
+    if (rc) return rc;
+    EGPU_CUDA_TRY(ctx, D.idx.alloc((size_t)n * gk));
+    const int grid = (int)std::max(1LL, std::min(((long long)n * gk + 255) / 256, (long long)ctx->num_sms * 32));
+    if (lower)
+      k_range_index<true><<<grid, 256, 0, ctx->stream>>>(n, bs, best_per, gk, best_per + ext, D.row.p, D.slot.p,
+                                                         D.ext_ptr.p, ds.p, A->ilu_rows.p, A->ilu_cols.p,
+                                                         A->ilu_diag.p, D.idx.p);
+    else
+      k_range_index<false><<<grid, 256, 0, ctx->stream>>>(n, bs, best_per, gk, best_per + ext, D.row.p, D.slot.p,
+                                                          D.ext_ptr.p, ds.p, A->ilu_rows.p, A->ilu_cols.p,
+                                                          A->ilu_diag.p, D.idx.p);
+    ctx->launches++;
+    EGPU_CUDA_TRY(ctx, cudaGetLastError());
+    EGPU_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    return EGPU_OK;
+  };
+  int rc = upload(best_lo, true, S.rg_lo);
+  if (!rc) rc = upload(best_up, false, S.rg_up);
+  if (rc) return rc;
+  const int maxr = std::max(best_lo.max_rows, best_up.max_rows);
+  S.rg_rows = best_per;
+  S.rg_ext = ext;
+  S.rg_g = sh.g;
+  S.rg_k = sh.k;
+  S.rg_nt = (maxr * sh.g + 31) / 32 * 32;
+  S.rg_stage[0] = plan::range_record(maxr, gk, 8);
+  S.rg_stage[1] = plan::range_record(maxr, gk, 4);
+  S.rg_ok[0] = best_fit == 0;
+  S.rg_ok[1] = true;
+  return EGPU_OK;
+}
+
+bool range_use(const egpu_mat *A, int v) {
+  const int mode = tri_mode_env();
+  return A->tri.rg_rows > 0 && A->tri.rg_ok[v] && mode != 1 && mode != 2;
+}
+
+// The level records of a triangle (plan::RangeLevel) with the factors' values.  bs > 1: row k of a
+// node block takes column e of the block's out-of-block part times the inverse of the block's
+// unit lower triangle, or of its upper triangle with the inverted diagonal; bs == 1: L_ij, or
+// u_ii^-1 U_ij.
+template <typename VT, bool LOWER>
+__global__ void k_range_pack(int n, int bs, int per, int g, int gk, const int *__restrict__ row,
+                             const int *__restrict__ slot_lev, const int2 *__restrict__ lev,
+                             const long long *__restrict__ offset, const uint16_t *__restrict__ idx,
+                             const int *__restrict__ rows, const int *__restrict__ diag,
+                             const double *__restrict__ ilu, unsigned char *__restrict__ rec) {
+  const long long tot = (long long)n * gk;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
+    const int gs = (int)(q / gk), e = (int)(q % gk);
+    const int l = slot_lev[gs], s = gs % per;
+    const int2 L = lev[l];
+    unsigned char *R = rec + offset[l];
+    const int r = row[gs], kr = r % bs, r0 = r - kr, t = s - L.x;
+    const int beg0 = rows[r0], len = rows[r0 + 1] - beg0, e_lo = diag[r0] - beg0;
+    const int off = LOWER ? 0 : e_lo + bs, ne = LOWER ? e_lo : len - e_lo - bs;
+    double v = 0.0;
+    if (e < ne) {
+      if (bs == 1) {
+        v = ilu[beg0 + off + e];
+        if (!LOWER) v *= ilu[diag[r0]];
+      } else {
+        double m[TRI_BS_MAX];
+        for (int i = 0; i < bs; ++i) {
+          const int j = LOWER ? i : bs - 1 - i;  // rows in elimination order, up to this one
+          double w = ilu[beg0 + j * len + off + e];
+          const double *in = ilu + beg0 + j * len + e_lo;
+          for (int h = 0; h < i; ++h) w -= in[LOWER ? h : bs - 1 - h] * m[h];
+          if (!LOWER) w *= in[j];
+          m[i] = w;
+          if (j == kr) {
+            v = w;
+            break;
+          }
+        }
+      }
+    }
+    const int at = plan::range_entry_at(L.y, g, t, e);
+    reinterpret_cast<uint16_t *>(R + plan::range_idx_at(L.y))[at] = idx[q];
+    reinterpret_cast<VT *>(R + plan::range_val_at(L.y, gk))[at] = (VT)v;
+    if (e == 0) {
+      reinterpret_cast<int *>(R)[4 + t] = r;
+      if (t == 0) *reinterpret_cast<int4 *>(R) = make_int4(L.x, L.y, 0, 0);
+    }
+  }
+}
+
+template <typename VT>
+static int range_pack_as(egpu_mat *A, int v) {
+  egpu_ctx *ctx = A->ctx;
+  const TriSchedule &S = A->tri;
+  const int gk = S.rg_g * S.rg_k;
+  const int grid = (int)std::max(1LL, std::min(((long long)A->n * gk + 255) / 256, (long long)ctx->num_sms * 32));
+  EGPU_CUDA_TRY(ctx, A->rg_lo_rec[v].alloc(S.rg_lo.bytes[v]));
+  EGPU_CUDA_TRY(ctx, A->rg_up_rec[v].alloc(S.rg_up.bytes[v]));
+  k_range_pack<VT, true><<<grid, 256, 0, ctx->stream>>>(
+      A->n, S.bs, S.rg_rows, S.rg_g, gk, S.rg_lo.row.p, S.rg_lo.slot_lev.p, S.rg_lo.lev.p, S.rg_lo.offset[v].p,
+      S.rg_lo.idx.p, A->ilu_rows.p, A->ilu_diag.p, A->ilu.p, A->rg_lo_rec[v].p);
+  k_range_pack<VT, false><<<grid, 256, 0, ctx->stream>>>(
+      A->n, S.bs, S.rg_rows, S.rg_g, gk, S.rg_up.row.p, S.rg_up.slot_lev.p, S.rg_up.lev.p, S.rg_up.offset[v].p,
+      S.rg_up.idx.p, A->ilu_rows.p, A->ilu_diag.p, A->ilu.p, A->rg_up_rec[v].p);
+  ctx->launches += 2;
+  EGPU_CUDA_TRY(ctx, cudaGetLastError());
+  A->rg_packed[v] = true;
+  return EGPU_OK;
+}
+
+int range_pack(egpu_mat *A, int v) {
+  if (!range_use(A, v) || A->rg_packed[v]) return EGPU_OK;
+  return v == 0 ? range_pack_as<double>(A, v) : range_pack_as<float>(A, v);
 }
 
 }  // namespace egpu
