@@ -178,47 +178,59 @@ __global__ void k_backscale_x(int n, const double *__restrict__ xs, const double
 // (every row after the rows of its strictly lower part).  The warp runs the IKJ loop over
 // the rows k of its strictly lower part in ascending column order, each once it is done:
 // S_m /= u_kk, then S_j -= S_m * U_kj for the U entries of row k that fall in the row's
-// pattern (found by binary search in the row's columns).  Row k+1's U entries and u_kk are
-// loaded while row k's update runs.  Every entry of the row sees its updates in the
-// reference's order, so the factor is bit-identical to the sequential routine.  The U
-// diagonal stays un-inverted.
+// pattern (found by binary search in the row's columns).  Every entry of the row sees its
+// updates in the reference's order, so the factor is bit-identical to the sequential routine.
+// The U diagonal stays un-inverted.
+//
+// What bounds it is latency per dependency, 13 of them a row on a 27-point stencil.  The row
+// bounds of all dependencies of a round are loaded at once, and the U entries of the next four
+// while four are processed (fetched one by one, each cost two dependent L2 round trips); the
+// binary search has a fixed number of steps, so it runs in the shadow of the division.
 struct IluDep {
-  int dk, kend;
   int c0, c1;
   double v0, v1, ukk;
 };
 
-__device__ __forceinline__ void ilu_dep_fetch(IluDep &d, int k, const int *__restrict__ rows,
-                                              const int *__restrict__ cols, const int *__restrict__ diag,
+// the U entries of a row (row bounds dk, kend) held by a lane: two, or one where no row is longer
+// than 32
+template <bool TWO>
+__device__ __forceinline__ void ilu_dep_fetch(IluDep &d, int dk, int kend, const int *__restrict__ cols,
                                               const double *ilu, int lane) {
-  d.dk = __ldg(diag + k);
-  d.kend = __ldg(rows + k + 1);
-  const int l0 = d.dk + 1 + lane, l1 = l0 + 32;
-  d.c0 = l0 < d.kend ? __ldg(cols + l0) : -1;
-  d.c1 = l1 < d.kend ? __ldg(cols + l1) : -1;
-  d.v0 = l0 < d.kend ? __ldcg(ilu + l0) : 0.0;
-  d.v1 = l1 < d.kend ? __ldcg(ilu + l1) : 0.0;
-  d.ukk = __ldcg(ilu + d.dk);
+  const int l0 = dk + 1 + lane, l1 = l0 + 32;
+  d.c0 = l0 < kend ? __ldg(cols + l0) : -1;
+  d.v0 = l0 < kend ? __ldcg(ilu + l0) : 0.0;
+  d.c1 = TWO && l1 < kend ? __ldg(cols + l1) : -1;
+  d.v1 = TWO && l1 < kend ? __ldcg(ilu + l1) : 0.0;
+  d.ukk = __ldcg(ilu + dk);
 }
 
-// position of column j among the row's sorted columns Cc[0..len), -1 if absent
+// position of column j among the row's sorted columns, -1 if absent.  STEPS > 0: Cc holds
+// 2^STEPS columns, padded with INT_MAX; else Cc[0..len).
+template <int STEPS>
 __device__ __forceinline__ int ilu_find(const int *Cc, int len, int j) {
-  int lo = 0, hi = len - 1;
-  while (lo <= hi) {
-    const int mid = (lo + hi) >> 1;
-    const int cm = Cc[mid];
-    if (cm == j) return mid;
-    if (cm < j)
-      lo = mid + 1;
-    else
-      hi = mid - 1;
+  if constexpr (STEPS > 0) {
+    int lo = 0;
+#pragma unroll
+    for (int q = STEPS - 1; q >= 0; --q) lo += Cc[lo + (1 << q)] <= j ? 1 << q : 0;
+    return j >= 0 && Cc[lo] == j ? lo : -1;
+  } else {
+    int lo = 0, hi = len - 1;
+    while (lo <= hi) {
+      const int mid = (lo + hi) >> 1;
+      const int cm = Cc[mid];
+      if (cm == j) return mid;
+      if (cm < j)
+        lo = mid + 1;
+      else
+        hi = mid - 1;
+    }
+    return -1;
   }
-  return -1;
 }
 
-// MAXROW > 0: the row's values and columns are staged in shared memory (rows of at most
-// MAXROW entries).  MAXROW == 0: rows of any length; the row is updated in place in its own
-// slots of the output (private to the warp until its done flag is published) and the
+// MAXROW > 0 (a power of two): the row's values and columns are staged in shared memory (rows of
+// at most MAXROW entries).  MAXROW == 0: rows of any length; the row is updated in place in its
+// own slots of the output (private to the warp until its done flag is published) and the
 // binary searches run over its columns in global memory.
 template <int MAXROW>
 __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restrict__ rows,
@@ -228,6 +240,9 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
                                                      const double *__restrict__ A, double *ilu,
                                                      int *done, int *err) {
   constexpr int SR = MAXROW > 0 ? MAXROW : 1;
+  constexpr int STEPS = MAXROW == 32 ? 5 : MAXROW == 128 ? 7 : MAXROW == 256 ? 8 : 0;
+  constexpr bool TWO = MAXROW != 32;
+  constexpr int CH = TWO ? 2 : 4;  // dependencies fetched together
   __shared__ double S_all[8][SR];
   __shared__ int C_all[8][SR];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -246,10 +261,9 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
     }
     double *S = MAXROW > 0 ? S_all[wib] : ilu + beg;
     const int *Cc = MAXROW > 0 ? C_all[wib] : cols + beg;
-    for (int t = lane; t < len; t += 32) {
-      S[t] = A[beg + t];
-      if (MAXROW > 0) C_all[wib][t] = cols[beg + t];
-    }
+    for (int t = lane; t < len; t += 32) S[t] = A[beg + t];
+    if (MAXROW > 0)
+      for (int t = lane; t < SR; t += 32) C_all[wib][t] = t < len ? cols[beg + t] : 0x7fffffff;
     __syncwarp();
     // The dependencies are taken in rounds: the 32 lanes poll the done flags of the next 32
     // rows of the strictly lower part at once (acquire), and the leading run of finished
@@ -258,8 +272,15 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
     // wait.
     unsigned long long t0 = 0;
     unsigned int spin = 0;
+    int mh = -1, dk = 0, ke = 0;  // lane's dependency m0 + lane: bounds of its U part (of round mh)
     for (int m0 = 0; m0 < nl;) {
       const int mp = m0 + lane;
+      if (mh != m0) {
+        mh = m0;
+        const int k = mp < nl ? Cc[mp] : i;
+        dk = __ldg(diag + k);
+        ke = __ldg(rows + k + 1);
+      }
       const bool ok = mp >= nl || ld_acquire_s32(done + Cc[mp]) != 0;
       const unsigned int mask = __ballot_sync(0xffffffffu, ok);
       __syncwarp();
@@ -278,29 +299,42 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
         continue;
       }
       const int m1 = min(nl, m0 + ready);
-      IluDep nxt;
-      ilu_dep_fetch(nxt, Cc[m0], rows, cols, diag, ilu, lane);
-      for (int m = m0; m < m1; ++m) {
-        const IluDep cur = nxt;
-        if (m + 1 < m1) ilu_dep_fetch(nxt, Cc[m + 1], rows, cols, diag, ilu, lane);
-        double sk = S[m];
-        if (sk == 0.0) continue;
-        if (fabs(cur.ukk) > EGPU_AEPS) sk = sk / cur.ukk;
-        __syncwarp();
-        if (lane == 0) S[m] = sk;
-        if (cur.c0 >= 0) {
-          const int pos = ilu_find(Cc, len, cur.c0);
-          if (pos >= 0) S[pos] = __dsub_rn(S[pos], __dmul_rn(sk, cur.v0));
+      IluDep nxt[CH];
+      auto fetch = [&](int mb) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          const int h = min(mb + u, m1 - 1) - m0;  // past the end: the last one again, unused
+          ilu_dep_fetch<TWO>(nxt[u], __shfl_sync(0xffffffffu, dk, h), __shfl_sync(0xffffffffu, ke, h), cols, ilu, lane);
         }
-        if (cur.c1 >= 0) {
-          const int pos = ilu_find(Cc, len, cur.c1);
-          if (pos >= 0) S[pos] = __dsub_rn(S[pos], __dmul_rn(sk, cur.v1));
+      };
+      fetch(m0);
+      for (int mb = m0; mb < m1; mb += CH) {
+        IluDep cur[CH];
+#pragma unroll
+        for (int u = 0; u < CH; ++u) cur[u] = nxt[u];
+        if (mb + CH < m1) fetch(mb + CH);
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          const int m = mb + u;
+          if (m >= m1) break;
+          double sk = S[m];
+          if (sk == 0.0) continue;
+          const int p0 = ilu_find<STEPS>(Cc, len, cur[u].c0);
+          const int p1 = TWO ? ilu_find<STEPS>(Cc, len, cur[u].c1) : -1;
+          if (fabs(cur[u].ukk) > EGPU_AEPS) sk = sk / cur[u].ukk;
+          __syncwarp();
+          if (lane == 0) S[m] = sk;
+          if (p0 >= 0) S[p0] = __dsub_rn(S[p0], __dmul_rn(sk, cur[u].v0));
+          if (p1 >= 0) S[p1] = __dsub_rn(S[p1], __dmul_rn(sk, cur[u].v1));
+          if (TWO) {
+            const int de = __shfl_sync(0xffffffffu, dk, m - m0), ee = __shfl_sync(0xffffffffu, ke, m - m0);
+            for (int l = de + 65 + lane; l < ee; l += 32) {
+              const int pos = ilu_find<STEPS>(Cc, len, cols[l]);
+              if (pos >= 0) S[pos] = __dsub_rn(S[pos], __dmul_rn(sk, __ldcg(ilu + l)));
+            }
+          }
+          __syncwarp();
         }
-        for (int l = cur.dk + 65 + lane; l < cur.kend; l += 32) {
-          const int pos = ilu_find(Cc, len, cols[l]);
-          if (pos >= 0) S[pos] = __dsub_rn(S[pos], __dmul_rn(sk, __ldcg(ilu + l)));
-        }
-        __syncwarp();
       }
       __syncwarp();
       m0 = m1;
@@ -308,10 +342,8 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
     if (MAXROW > 0)
       for (int t = lane; t < len; t += 32) ilu[beg + t] = S[t];
     __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      st_release_s32(done + i, 1);
-    }
+    // the release orders the whole warp's stores (they happen before it through the warp barrier)
+    if (lane == 0) st_release_s32(done + i, 1);
   }
 }
 
