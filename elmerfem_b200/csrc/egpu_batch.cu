@@ -1510,7 +1510,7 @@ static int batch_prepare(egpu_batch *B, int slot, const double *b_dev) {
   const int n = A->n;
   int rc = reset_sync(ctx);
   if (rc) return rc;
-  rc = scale_matrix(A, B->prm.scale_system != 0);
+  rc = scale_matrix(A, B->prm.scale_system != 0, is_ilu(B->prm.precond), true);
   if (rc) return rc;
   const long long ldw = A->ldw;
   double *W = A->work.p;

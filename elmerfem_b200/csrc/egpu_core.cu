@@ -53,36 +53,58 @@ __global__ void k_scale_diag(int n, const int *__restrict__ rows, const int *__r
   }
 }
 
-// a_ij * (D_i * D_j) (SolverUtils.src:6570-6575); also the scaled diagonal for Jacobi
-__global__ void k_scale_values(int n, const int *__restrict__ rows, const int *__restrict__ cols,
-                               const int *__restrict__ diag, const double *__restrict__ vals,
-                               const double *__restrict__ D, double *__restrict__ out,
-                               double *__restrict__ dvals) {
-  const int lane = threadIdx.x & 7;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; i < n; i += (gridDim.x * blockDim.x) >> 3) {
-    const double di = D[i];
-    for (int k = rows[i] + lane; k < rows[i + 1]; k += 8) out[k] = vals[k] * (di * D[cols[k]]);
-    if (lane == 0) dvals[i] = diag[i] >= 0 ? vals[diag[i]] * (di * di) : 0.0;
-  }
-}
-
-// scaled values in SELL-32 order (thread per row; padding entries 0)
-__global__ void k_sell_scale(int n, int nslices, const int *__restrict__ rows, const int *__restrict__ cols,
-                             const double *__restrict__ vals, const double *__restrict__ D,
-                             const int *__restrict__ sell_ptr, const int *__restrict__ sell_w,
-                             double *__restrict__ out) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nslices * 32; r += gridDim.x * blockDim.x) {
-    const int sl = r >> 5, lane = r & 31;
-    const int w = sell_w[sl];
-    double *o = out + sell_ptr[sl] + lane;
+// a_ij * (D_i * D_j) (SolverUtils.src:6570-6575) into the SELL-32 layout (padding entries 0), with
+// the scaled diagonal for Jacobi; optionally the same in CRS order (the ILU factorisation's
+// input) and FP32 copies of values and diagonal (the inner solver's).  One warp per slice: a
+// row's entries are read side by side and leave through a transposed tile in shared memory, so
+// reads and writes are whole sectors and every entry is scaled once.  128^3: 0.40 ms; a pass per
+// output, the SELL one with a thread per row, 0.64 ms.
+constexpr int SCALE_WARPS = 4;
+template <bool CRS, bool F32>
+__global__ void __launch_bounds__(SCALE_WARPS * 32) k_scale_sell(
+    int n, int nslices, const int *__restrict__ rows, const int *__restrict__ cols, const int *__restrict__ diag,
+    const double *__restrict__ vals, const double *__restrict__ D, const int *__restrict__ sell_ptr,
+    const int *__restrict__ sell_w, double *__restrict__ sell, double *__restrict__ dvals, double *__restrict__ crs,
+    float *__restrict__ sell32, float *__restrict__ dvals32) {
+  __shared__ double tile[SCALE_WARPS][32][33];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  for (int sl = blockIdx.x * SCALE_WARPS + wib; sl < nslices; sl += gridDim.x * SCALE_WARPS) {
+    const int r = (sl << 5) + lane, w = __ldg(sell_w + sl);
+    const size_t out = (size_t)__ldg(sell_ptr + sl) + lane;
     int beg = 0, len = 0;
     double dr = 0.0;
     if (r < n) {
-      beg = rows[r];
-      len = rows[r + 1] - beg;
-      dr = D[r];
+      beg = __ldg(rows + r);
+      len = __ldg(rows + r + 1) - beg;
+      dr = __ldg(D + r);
+      const int dg = __ldg(diag + r);
+      const double d = dg >= 0 ? vals[dg] * (dr * dr) : 0.0;
+      dvals[r] = d;
+      if (F32) dvals32[r] = (float)d;
     }
-    for (int k = 0; k < w; ++k) o[32 * k] = k < len ? vals[beg + k] * (dr * D[cols[beg + k]]) : 0.0;
+    for (int k0 = 0; k0 < w; k0 += 32) {
+#pragma unroll 8
+      for (int q = 0; q < 32; ++q) {  // row q of the slice, entries k0 + lane
+        const int b = __shfl_sync(0xffffffffu, beg, q), l = __shfl_sync(0xffffffffu, len, q);
+        const double dq = __shfl_sync(0xffffffffu, dr, q);
+        double v = 0.0;
+        if (k0 + lane < l) {
+          const int e = b + k0 + lane;
+          v = vals[e] * (dq * __ldg(D + __ldg(cols + e)));
+          if (CRS) crs[e] = v;
+        }
+        tile[wib][lane][q] = v;
+      }
+      __syncwarp();
+      const int kn = min(32, w - k0);
+#pragma unroll 4
+      for (int k = 0; k < kn; ++k) {
+        const double v = tile[wib][k][lane];
+        sell[out + ((size_t)(k0 + k) << 5)] = v;
+        if (F32) sell32[out + ((size_t)(k0 + k) << 5)] = (float)v;
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -620,26 +642,42 @@ int read_err(egpu_ctx *ctx, int *err) {
   return EGPU_OK;
 }
 
-// Scale: scaled = D A D, dvals = diag(scaled), D = DiagScaling (not yet times ||Db||)
-int scale_matrix(egpu_mat *A, bool scale_system) {
+// Scale: D = DiagScaling (not yet times ||Db||), sell_vals = D A D, dvals = its diagonal; crs:
+// also in CRS order (scaled), f32: also the FP32 copies of the inner solver
+int scale_matrix(egpu_mat *A, bool scale_system, bool crs, bool f32) {
   egpu_ctx *ctx = A->ctx;
   const int n = A->n;
-  EGPU_CUDA_TRY(ctx, A->scaled.alloc(A->nnz));
+  if (crs) EGPU_CUDA_TRY(ctx, A->scaled.alloc(A->nnz));
   EGPU_CUDA_TRY(ctx, A->dscale.alloc(n));
   EGPU_CUDA_TRY(ctx, A->work.alloc((size_t)13 * A->ldw));
+  EGPU_CUDA_TRY(ctx, A->sell_vals.alloc(A->sell_nnz));
+  if (f32) {
+    EGPU_CUDA_TRY(ctx, A->work32.alloc((size_t)14 * A->ldw));
+    EGPU_CUDA_TRY(ctx, A->sell_vals32.alloc(A->sell_nnz));
+  }
   double *dvals = A->work.p + (size_t)11 * A->ldw;
+  float *dvals32 = f32 ? A->work32.p + (size_t)13 * A->ldw : nullptr;
   if (scale_system) {
     k_scale_diag<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(n, A->rows.p, A->diag.p, A->values.p, A->dscale.p);
   } else {
     k_fill64<<<grid_for(ctx, n), 256, 0, ctx->stream>>>((unsigned long long *)A->dscale.p,
                                                          0x3FF0000000000000ull, n);
   }
-  k_scale_values<<<grid_for(ctx, (long long)n * 8), 256, 0, ctx->stream>>>(
-      n, A->rows.p, A->cols.p, A->diag.p, A->values.p, A->dscale.p, A->scaled.p, dvals);
-  EGPU_CUDA_TRY(ctx, A->sell_vals.alloc(A->sell_nnz));
-  k_sell_scale<<<grid_for(ctx, (long long)A->nslices * 32), 256, 0, ctx->stream>>>(
-      n, A->nslices, A->rows.p, A->cols.p, A->values.p, A->dscale.p, A->sell_ptr.p, A->sell_w.p, A->sell_vals.p);
-  ctx->launches += 3;
+  const int grid = std::max(1, std::min((A->nslices + SCALE_WARPS - 1) / SCALE_WARPS, ctx->num_sms * 12));
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, SCALE_WARPS * 32, 0, ctx->stream>>>(n, A->nslices, A->rows.p, A->cols.p, A->diag.p, A->values.p,
+                                                       A->dscale.p, A->sell_ptr.p, A->sell_w.p, A->sell_vals.p, dvals,
+                                                       A->scaled.p, A->sell_vals32.p, dvals32);
+  };
+  if (crs && f32)
+    launch(k_scale_sell<true, true>);
+  else if (crs)
+    launch(k_scale_sell<true, false>);
+  else if (f32)
+    launch(k_scale_sell<false, true>);
+  else
+    launch(k_scale_sell<false, false>);
+  ctx->launches += 2;
   EGPU_CUDA_TRY(ctx, cudaGetLastError());
   return EGPU_OK;
 }
@@ -1139,6 +1177,25 @@ static int run_krylov(egpu_mat *A, const KArgs<VT> &a0, int method, bool offs) {
   return launch_bicgstab(ctx, a, offs, form, smem);
 }
 
+// Loads the Krylov kernel a solve is about to launch (kernels are loaded on first use) without
+// launching it, so that a matrix's first timed solve by a path does not carry that.
+template <typename VT>
+static int krylov_load(egpu_mat *A, const egpu_params *prm, int sweeps) {
+  KArgs<VT> a{};
+  a.precond = is_ilu(prm->precond) ? EGPU_PREC_ILU0 : prm->precond;
+  if (a.precond == EGPU_PREC_ILU0) {
+    if (!A->tri_built) return EGPU_OK;  // the matrix's first factorisation: not timed
+    set_tri(a, A);
+    if (range_use(A, sizeof(VT) == 8 ? 0 : 1)) {
+      a.rg_rows = A->tri.rg_rows;
+      a.tri_cta = 0;
+    }
+    a.sweeps_l = a.sweeps_u = sweeps;
+    if (sweeps > 0) a.tri_cta = a.rg_rows = 0;
+  }
+  return run_krylov<VT>(A, a, prm->method, A->sell_c16.p != nullptr);
+}
+
 // stored vectors of GCR (2 (m-1) directions) / BiCGStab(l) (r_0..r_l, u_0..u_l, shadow, x,
 // xp, bp, t): allocated per matrix, refused when they would take more than half the free
 // device memory
@@ -1178,11 +1235,14 @@ int solve_fp64(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_param
   const int n = A->n;
   int rc = ensure_ctx_scratch(ctx);
   if (rc) return rc;
+  // buffers and kernels of this path before the clock starts (see egpu_iter_solve_dev)
+  if (is_ilu(prm->precond) && (rc = range_alloc(A, 0))) return rc;
+  if ((rc = krylov_load<double>(A, prm, 0))) return rc;
   EGPU_CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
   rc = reset_sync(ctx);
   if (rc) return rc;
   const bool sc = prm->scale_system != 0;
-  rc = scale_matrix(A, sc);
+  rc = scale_matrix(A, sc, is_ilu(prm->precond), false);
   if (rc) return rc;
   double *W = A->work.p;
   const long long ldw = A->ldw;
@@ -1220,7 +1280,6 @@ int solve_fp64(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_param
   a.cols = A->cols.p;
   a.diag = A->diag.p;
   a.cols16 = nullptr;
-  a.vals = A->scaled.p;
   set_sell(a, A, A->sell_vals.p, A->sell_c16.p != nullptr);
   a.ilu = A->ilu.p;
   a.dvals = dvals;
@@ -1295,10 +1354,14 @@ int solve_fp64(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_param
 // -------------------------------------------------------------------------------------
 // mixed precision: FP32 inner Krylov inside FP64 iterative refinement
 
-// r = b - A x (FP64) and partial ||r||^2
-template <int LPR>
-__global__ void __launch_bounds__(EGPU_BLOCK) k_residual(int n, const int *__restrict__ rows,
-                                                         const int *__restrict__ cols,
+// r = b - A x (FP64, rows summed in CRS order as CRS_MatrixVectorProd) and partial ||r||^2, on the
+// SELL copy: a warp per slice, column offsets shared where the slice's rows share them (8.5
+// bytes an entry instead of CRS's 12).  Bound by its bytes; 128^3: 197 -> 128 us, 3.8 TB/s.
+__global__ void __launch_bounds__(EGPU_BLOCK) k_residual(int n, int nslices, const int *__restrict__ sell_ptr,
+                                                         const int *__restrict__ sell_w,
+                                                         const int *__restrict__ scols,
+                                                         const int *__restrict__ sell_cptr,
+                                                         const int16_t *__restrict__ scolsc,
                                                          const double *__restrict__ vals,
                                                          const double *__restrict__ b,
                                                          const double *__restrict__ x,
@@ -1306,19 +1369,29 @@ __global__ void __launch_bounds__(EGPU_BLOCK) k_residual(int n, const int *__res
                                                          double *__restrict__ partials) {
   __shared__ double sm[32];
   const int lane = threadIdx.x & 31;
-  const int sl = lane & (LPR - 1);
-  const unsigned submask = (LPR == 32) ? 0xffffffffu : (((1u << LPR) - 1u) << (lane & ~(LPR - 1)));
-  const int gsub = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / LPR);
-  const int nsub = (int)((long long)gridDim.x * blockDim.x / LPR);
+  const int gw = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nw = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   double acc[1] = {0.0};
-  for (int row = gsub; row < n; row += nsub) {
-    const int beg = __ldg(rows + row), end = __ldg(rows + row + 1);
-    double s = 0;
-#pragma unroll 4
-    for (int j = beg + sl; j < end; j += LPR) s += __ldcs(vals + j) * __ldcg(x + __ldcs(cols + j));
-#pragma unroll
-    for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(submask, s, off, LPR);
-    if (sl == 0) {
+  for (int sl = gw; sl < nslices; sl += nw) {
+    const int row = (sl << 5) + lane, w = __ldg(sell_w + sl);
+    const double *v = vals + __ldg(sell_ptr + sl) + lane;
+    const int cp = scolsc ? __ldg(sell_cptr + sl) : 0;
+    double s = 0.0;
+    if (cp < 0) {
+      const int16_t *co = scolsc + (-cp - 1);
+      for (int k0 = 0; k0 < w; k0 += 32) {
+        const int kn = min(32, w - k0);
+        const int offl = lane < kn ? (int)__ldg(co + k0 + lane) : 0;
+#pragma unroll 8
+        for (int k = 0; k < kn; ++k)
+          s = __dadd_rn(s, __dmul_rn(__ldcs(v + ((k0 + k) << 5)), __ldg(x + row + __shfl_sync(0xffffffffu, offl, k))));
+      }
+    } else {
+      const int *c = scols + __ldg(sell_ptr + sl) + lane;
+#pragma unroll 8
+      for (int k = 0; k < w; ++k) s = __dadd_rn(s, __dmul_rn(__ldcs(v + (k << 5)), __ldg(x + __ldcs(c + (k << 5)))));
+    }
+    if (row < n) {
       const double ri = b[row] - s;
       r[row] = ri;
       acc[0] += ri * ri;
@@ -1355,19 +1428,6 @@ __global__ void k_refine_update(int n, const float *__restrict__ d, const double
     x[i] += rn * (double)d[i];
 }
 
-template <typename K>
-static void launch_lpr_residual(egpu_ctx *ctx, int lpr, int grid, int n, const int *rows, const int *cols,
-                                const double *vals, const double *b, const double *x, double *r,
-                                double *partials) {
-  switch (lpr) {
-    case 4: k_residual<4><<<grid, EGPU_BLOCK, 0, ctx->stream>>>(n, rows, cols, vals, b, x, r, partials); break;
-    case 8: k_residual<8><<<grid, EGPU_BLOCK, 0, ctx->stream>>>(n, rows, cols, vals, b, x, r, partials); break;
-    case 16: k_residual<16><<<grid, EGPU_BLOCK, 0, ctx->stream>>>(n, rows, cols, vals, b, x, r, partials); break;
-    default: k_residual<32><<<grid, EGPU_BLOCK, 0, ctx->stream>>>(n, rows, cols, vals, b, x, r, partials); break;
-  }
-  ctx->launches++;
-}
-
 int krylov_fp64_scaled(egpu_mat *A, const double *bs, double *xs, const egpu_params *prm, int *info,
                        int *iters, double *residual) {
   egpu_ctx *ctx = A->ctx;
@@ -1379,7 +1439,6 @@ int krylov_fp64_scaled(egpu_mat *A, const double *bs, double *xs, const egpu_par
   a.rows = A->rows.p;
   a.cols = A->cols.p;
   a.diag = A->diag.p;
-  a.vals = A->scaled.p;
   set_sell(a, A, A->sell_vals.p, A->sell_c16.p != nullptr);
   a.ilu = A->ilu.p;
   a.dvals = A->work.p + (size_t)11 * A->ldw;
@@ -1413,8 +1472,8 @@ int krylov_fp64_scaled(egpu_mat *A, const double *bs, double *xs, const egpu_par
   return EGPU_OK;
 }
 
-// FP32 copies of the scaled matrix, its diagonal and the ILU0 factors; int16 column
-// offsets when every |col - row| < 32768.
+// FP32 copies of the ILU0 factors (the scaled matrix's are scale_matrix's); int16 column offsets
+// when every |col - row| < 32768.
 // entries of d that are not exactly 1.0f (the scaled matrix's diagonal in FP32)
 __global__ void k_count_not_one(const float *__restrict__ d, int n, unsigned int *cnt) {
   unsigned int c = 0;
@@ -1426,12 +1485,6 @@ __global__ void k_count_not_one(const float *__restrict__ d, int n, unsigned int
 static int prepare_fp32(egpu_mat *A, bool with_ilu, bool sweeps) {
   egpu_ctx *ctx = A->ctx;
   const int n = A->n;
-  EGPU_CUDA_TRY(ctx, A->work32.alloc((size_t)14 * A->ldw));
-  k_to_f32<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(A->work.p + (size_t)11 * A->ldw,
-                                                       A->work32.p + (size_t)13 * A->ldw, n);
-  EGPU_CUDA_TRY(ctx, A->sell_vals32.alloc(A->sell_nnz));
-  k_to_f32<<<grid_for(ctx, A->sell_nnz), 256, 0, ctx->stream>>>(A->sell_vals.p, A->sell_vals32.p, A->sell_nnz);
-  ctx->launches += 2;
   if (with_ilu) {
     EGPU_CUDA_TRY(ctx, A->ilu32.alloc(A->ilu_nnz));
     k_to_f32<<<grid_for(ctx, A->ilu_nnz), 256, 0, ctx->stream>>>(A->ilu.p, A->ilu32.p, A->ilu_nnz);
@@ -1461,11 +1514,25 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
   const int n = A->n;
   int rc = ensure_ctx_scratch(ctx);
   if (rc) return rc;
+  // ILU0 by Jacobi sweeps in the FP32 inner BiCGStab (the count egpu_iter_solve_dev chose)
+  const int sweeps = std::max(0, std::min(prm->ilu_sweeps, 16));
+  const bool ask_sweeps = sweeps > 0 && prm->method == EGPU_BICGSTAB && prm->precond == EGPU_PREC_ILU0 && prm->ilu_order == 0;
+  // buffers and kernels of this path before the clock starts (see egpu_iter_solve_dev)
+  if (ask_sweeps) {
+    EGPU_CUDA_TRY(ctx, A->ilu_sell32.alloc(A->sell_nnz));
+    EGPU_CUDA_TRY(ctx, A->ilu_dinv32.alloc(n));
+    cudaFuncAttributes fa;
+    EGPU_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, k_sell_gather32));
+    EGPU_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, k_gather_diag32));
+  } else if (is_ilu(prm->precond) && (rc = range_alloc(A, 1))) {
+    return rc;
+  }
+  if ((rc = krylov_load<float>(A, prm, ask_sweeps ? sweeps : 0))) return rc;
   EGPU_CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
   rc = reset_sync(ctx);
   if (rc) return rc;
   const bool sc = prm->scale_system != 0;
-  rc = scale_matrix(A, sc);
+  rc = scale_matrix(A, sc, is_ilu(prm->precond), true);
   if (rc) return rc;
   double *W = A->work.p;
   const long long ldw = A->ldw;
@@ -1484,10 +1551,7 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
     rc = precond_factor(A, prm);
     if (rc) return rc;
   }
-  // ILU0 by Jacobi sweeps in the FP32 inner BiCGStab (the count egpu_iter_solve_dev chose)
-  const int sweeps = std::max(0, std::min(prm->ilu_sweeps, 16));
-  const bool use_sweeps = sweeps > 0 && prm->method == EGPU_BICGSTAB && prm->precond == EGPU_PREC_ILU0 &&
-                          A->ilu_order == 0 && A->ilu_nnz == A->nnz;
+  const bool use_sweeps = ask_sweeps && A->ilu_order == 0 && A->ilu_nnz == A->nnz;
   rc = prepare_fp32(A, ilu, use_sweeps);
   if (rc) return rc;
   float *W32 = A->work32.p;
@@ -1506,9 +1570,7 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
   const bool unit_diag = prm->precond == EGPU_PREC_DIAGONAL && hf[1] == 0;
   egpu_result r{};
   double *norms = (double *)(ctx->sync.p + 32);
-  const int lpr = pick_lpr(A);
-  const int rgrid = std::min(1024, (int)std::min<long long>(((long long)n * lpr + EGPU_BLOCK - 1) / EGPU_BLOCK,
-                                                           (long long)ctx->num_sms * 4));
+  const int rgrid = std::max(1, std::min(std::min(1024, ctx->num_sms * 4), (A->nslices * 32 + EGPU_BLOCK - 1) / EGPU_BLOCK));
   // ||bs||: 1 after scaling with the right-hand-side normalisation, else ||b||
   double bnorm_s = 1.0;
   if (!sc) {
@@ -1531,7 +1593,10 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
     r.info = EGPU_HUTI_CONVERGENCE;
   } else {
     while (true) {
-      launch_lpr_residual<int>(ctx, lpr, rgrid, n, A->rows.p, A->cols.p, A->scaled.p, bs, xs, rr, ctx->partials.p);
+      k_residual<<<rgrid, EGPU_BLOCK, 0, ctx->stream>>>(n, A->nslices, A->sell_ptr.p, A->sell_w.p, A->sell_cols.p,
+                                                        A->sell_cptr.p, A->sell_csc.p, A->sell_vals.p, bs, xs, rr,
+                                                        ctx->partials.p);
+      ctx->launches++;
       k_residual_cast<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(n, rgrid, ctx->partials.p, rr, r32, norms);
       ctx->launches++;
       double hn[1];
@@ -1570,7 +1635,6 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
       a.cols = A->cols.p;
       a.diag = A->diag.p;
       a.cols16 = A->cols16.p;
-      a.vals = nullptr;  // the FP32 kernels read the SELL copy only
       set_sell(a, A, A->sell_vals32.p, A->sell_c16.p != nullptr);
       a.ilu = A->ilu32.p;
       a.dvals = dv32;
@@ -2377,7 +2441,7 @@ extern "C" int egpu_ilu_build(egpu_mat *A, int scale_system, int order) {
   cudaSetDevice(ctx->device);
   int rc = egpu::reset_sync(ctx);
   if (rc) return rc;
-  rc = egpu::scale_matrix(A, scale_system != 0);
+  rc = egpu::scale_matrix(A, scale_system != 0, true, false);
   if (rc) return rc;
   rc = egpu::ilu_factor(A, order);
   if (rc) return rc;
@@ -2400,7 +2464,7 @@ extern "C" int egpu_ilut_build(egpu_mat *A, int scale_system, double tol) {
   cudaSetDevice(ctx->device);
   int rc = egpu::reset_sync(ctx);
   if (rc) return rc;
-  rc = egpu::scale_matrix(A, scale_system != 0);
+  rc = egpu::scale_matrix(A, scale_system != 0, true, false);
   if (rc) return rc;
   rc = egpu::ilut_factor(A, tol);
   if (rc) return rc;

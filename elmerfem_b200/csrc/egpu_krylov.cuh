@@ -54,7 +54,6 @@ struct KArgs {
   int n;
   const int *rows, *cols, *diag;  // 0-based CRS
   const int16_t *cols16;          // col - row offsets (FP32 path, optional)
-  const VT *vals;                 // scaled matrix
   const VT *ilu;                  // ILU0 factors (inverted U diagonal)
   const VT *dvals;                // diagonal of the scaled matrix (Jacobi)
   const int *lower_order, *upper_order;

@@ -26,6 +26,7 @@ int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, si
     egpu_set_error(ctx, "persistent kernel does not fit on an SM");
     return EGPU_ERR_CUDA;
   }
+  if (args.nslices == 0) return EGPU_OK;  // the query above has loaded the kernel (krylov_load)
   bps = std::min(bps, 2048 / EGPU_KBLOCK);
   int grid = ctx->num_sms * bps;
   if (grid_out) *grid_out = grid;

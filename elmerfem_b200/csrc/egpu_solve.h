@@ -27,7 +27,7 @@ inline double inner_tol_of(const egpu_params *p) {
 
 int ensure_ctx_scratch(egpu_ctx *ctx);
 int reset_sync(egpu_ctx *ctx);
-int scale_matrix(egpu_mat *A, bool scale_system);
+int scale_matrix(egpu_mat *A, bool scale_system, bool crs, bool f32);
 int ensure_ilu_structure(egpu_mat *A, int order);
 int ensure_tri_schedule(egpu_mat *A);
 int ilu_factor(egpu_mat *A, int order);
@@ -64,6 +64,7 @@ int cta_fill_values(egpu_mat *A);
 // for it (v = 0 FP64, 1 FP32; once per factorisation), and whether a solve uses it
 int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vector<int> &cols,
                          const std::vector<int> &diag, const std::vector<int> &lev_lo, const std::vector<int> &lev_up);
+int range_alloc(egpu_mat *A, int v);
 int range_pack(egpu_mat *A, int v);
 bool range_use(const egpu_mat *A, int v);
 bool tri_prefer_node_blocks(int nlo, int nup, int bl, int bu, int n);

@@ -396,14 +396,28 @@ __global__ void k_range_pack(int n, int bs, int per, int g, int gk, const int *_
   }
 }
 
+// the record buffers of a precision, and its packing kernels loaded
+int range_alloc(egpu_mat *A, int v) {
+  if (!A->tri_built || !range_use(A, v)) return EGPU_OK;
+  egpu_ctx *ctx = A->ctx;
+  EGPU_CUDA_TRY(ctx, A->rg_lo_rec[v].alloc(A->tri.rg_lo.bytes[v]));
+  EGPU_CUDA_TRY(ctx, A->rg_up_rec[v].alloc(A->tri.rg_up.bytes[v]));
+  cudaFuncAttributes fa;
+  EGPU_CUDA_TRY(ctx, v == 0 ? cudaFuncGetAttributes(&fa, k_range_pack<double, true>)
+                            : cudaFuncGetAttributes(&fa, k_range_pack<float, true>));
+  EGPU_CUDA_TRY(ctx, v == 0 ? cudaFuncGetAttributes(&fa, k_range_pack<double, false>)
+                            : cudaFuncGetAttributes(&fa, k_range_pack<float, false>));
+  return EGPU_OK;
+}
+
 template <typename VT>
 static int range_pack_as(egpu_mat *A, int v) {
   egpu_ctx *ctx = A->ctx;
   const TriSchedule &S = A->tri;
   const int gk = S.rg_g * S.rg_k;
   const int grid = (int)std::max(1LL, std::min(((long long)A->n * gk + 255) / 256, (long long)ctx->num_sms * 32));
-  EGPU_CUDA_TRY(ctx, A->rg_lo_rec[v].alloc(S.rg_lo.bytes[v]));
-  EGPU_CUDA_TRY(ctx, A->rg_up_rec[v].alloc(S.rg_up.bytes[v]));
+  const int rc = range_alloc(A, v);
+  if (rc) return rc;
   k_range_pack<VT, true><<<grid, 256, 0, ctx->stream>>>(
       A->n, S.bs, S.rg_rows, S.rg_g, gk, S.rg_lo.row.p, S.rg_lo.slot_lev.p, S.rg_lo.lev.p, S.rg_lo.offset[v].p,
       S.rg_lo.idx.p, A->ilu_rows.p, A->ilu_diag.p, A->ilu.p, A->rg_lo_rec[v].p);
