@@ -420,17 +420,33 @@ struct Sentinel<float> {
 // solves, the ILU factorisation) doubled the set-up time of a large solve.  Returns false
 // when the kernel must unwind (error flag set by anyone).
 #define EGPU_ABORT_POLL 256u
-__device__ __forceinline__ bool grid_barrier(unsigned int *count, int *err, unsigned int &epoch) {
+// The counter and the error word are neighbours (words 0 and 1 of the control block), so one
+// 64-bit acquire load polls both; its result reaches the block through the closing barrier
+// (a separate read of the error word by every thread, and a fence after the poll, cost about
+// 0.6 us of the barrier).
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const void *p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+#ifdef EGPU_BARRIER_CALL
+static __device__ __noinline__
+#else
+__device__ __forceinline__
+#endif
+bool grid_barrier(unsigned int *count, int *err, unsigned int &epoch) {
   __syncthreads();
   epoch += 1;
+  int bad = 0;
   if (threadIdx.x == 0) {
     if (blockIdx.x == 0 && (epoch % EGPU_ABORT_POLL) == 0) egpu_poll_abort(err);
     const unsigned int target = epoch * gridDim.x;
     red_release_add_u32(count, 1u);
-    if (ld_acquire_u32(count) < target) {
+    unsigned long long w = ld_acquire_u64(count);
+    if ((unsigned int)w < target) {
       const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(err);
       unsigned int spins = 0;
-      while (ld_acquire_u32(count) < target) {
+      while ((unsigned int)(w = ld_acquire_u64(count)) < target) {
         if ((++spins & 63u) == 0) {
           // one block polls during long waits (block 0 may be the one still working)
           if ((spins & 1023u) == 0 && blockIdx.x == (gridDim.x > 1 ? 1u : 0u)) egpu_poll_abort(err);
@@ -441,11 +457,11 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *count, int *err, unsi
           }
         }
       }
+      if ((unsigned int)w < target) bad = 1;
     }
-    __threadfence();
+    bad |= (int)(w >> 32);
   }
-  __syncthreads();
-  return *(volatile int *)err == 0;
+  return __syncthreads_or(bad) == 0;
 }
 
 // Asynchronous global -> shared copies (cp.async, completion tracked per thread in
@@ -506,17 +522,37 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *smem /* >= 32
 }
 
 // Sum of partials[0..nb) read from L2 in a fixed order (same result in every block).
-__device__ __forceinline__ double reduce_partials(const double *partials, int nb, double *smem) {
+__device__ __forceinline__ double warp_partials(const double *partials, int nb) {
   double t = 0.0;
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x < 32) {
-    for (int i = lane; i < nb; i += 32) t += __ldcg(partials + i);
+  for (int i = threadIdx.x & 31; i < nb; i += 32) t += __ldcg(partials + i);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
-    if (lane == 0) smem[0] = t;
+  for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
+  return t;
+}
+__device__ __forceinline__ double reduce_partials(const double *partials, int nb, double *smem) {
+  if (threadIdx.x < 32) {
+    const double t = warp_partials(partials, nb);
+    if (threadIdx.x == 0) smem[0] = t;
   }
   __syncthreads();
-  t = smem[0];
+  const double t = smem[0];
   __syncthreads();
   return t;
+}
+// Several sums at once, one warp each: their loads and their chains of FP64 additions (about 60
+// cycles each) run side by side instead of one after another.
+template <int NV>
+__device__ __forceinline__ void reduce_partials_n(const double *const (&partials)[NV], int nb, double *smem,
+                                                  double (&out)[NV]) {
+  const int w = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (w == k) {
+      const double t = warp_partials(partials[k], nb);
+      if ((threadIdx.x & 31) == 0) smem[k] = t;
+    }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) out[k] = smem[k];
+  __syncthreads();
 }

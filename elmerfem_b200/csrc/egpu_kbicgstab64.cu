@@ -9,7 +9,8 @@ static int launch_form(egpu_ctx *ctx, KArgs<VT> &a, int form, size_t smem) {
     case TRI_CTA: return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, OFFS, TRI_CTA>, a, nullptr, smem);
     case TRI_RANGE7: return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, OFFS, TRI_RANGE7>, a, nullptr, smem);
     case TRI_RANGE10: return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, OFFS, TRI_RANGE10>, a, nullptr, smem);
-    default: return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, OFFS, TRI_SYNCFREE>, a, nullptr, smem);
+    default: return launch_coop(ctx, bicgstab_kernel<VT, TRI_TS, OFFS, TRI_SYNCFREE>, a, nullptr, smem,
+                                  a.precond == EGPU_PREC_ILU0 ? 0 : krylov_blocks(a.nslices));
   }
 }
 

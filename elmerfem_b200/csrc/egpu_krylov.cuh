@@ -1356,8 +1356,8 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
   // scale (rho is quadratic in the residual's scale, P linear)
   const bool resumed = a.resume && !a.true_residual;
   if (resumed) oldrho = a.carry[0] * a.ru_c;
+  rho = reduce_partials(a.partials + SLOT_RHO * nb, nb, sm);
   while (true) {
-    rho = reduce_partials(a.partials + SLOT_RHO * nb, nb, sm);
     if (!a.true_residual && k > 1) {
       // inner mode: recursive residual of x_{k-1}
       residual = sqrt(rr_prev) / rhsnorm;
@@ -1404,10 +1404,11 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
       store_partials(a, SLOT_RR, acc[1]);
     }
     if (!grid_barrier(a.bar, a.err, epoch)) return;
-    const double pq = reduce_partials(a.partials + SLOT_PQ * nb, nb, sm);
+    double pqrr[2];
+    reduce_partials_n<2>({a.partials + SLOT_PQ * nb, a.partials + SLOT_RR * nb}, nb, sm, pqrr);
+    const double pq = pqrr[0];
     if (a.true_residual && k > 1) {
-      const double rr = reduce_partials(a.partials + SLOT_RR * nb, nb, sm);
-      residual = sqrt(rr) / rhsnorm;
+      residual = sqrt(pqrr[1]) / rhsnorm;
       if (residual < a.tol) { info = EGPU_HUTI_CONVERGENCE; iters = k - 1; break; }
       if (k > a.maxit) { info = EGPU_HUTI_MAXITER; iters = k; break; }
     }
@@ -1495,9 +1496,12 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) cg_kernel(KArgs<VT> a) {
       }
     }
     if (!grid_barrier(a.bar, a.err, epoch)) return;
-    if (!a.true_residual) rr_prev = reduce_partials(a.partials + SLOT_RR2 * nb, nb, sm);
     oldrho = rho;
     ++k;
+    double rhrr[2];
+    reduce_partials_n<2>({a.partials + SLOT_RHO * nb, a.partials + SLOT_RR2 * nb}, nb, sm, rhrr);
+    rho = rhrr[0];
+    rr_prev = rhrr[1];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.out_i[0] = info;
@@ -1616,9 +1620,11 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
   }
   if (!a.true_residual) r0norm = sqrt(reduce_partials(a.partials + SLOT_RR2 * nb, nb, sm));
   while (true) {
-    rho = reduce_partials(a.partials + SLOT_RHO * nb, nb, sm);
+    double rhrr[2];
+    reduce_partials_n<2>({a.partials + SLOT_RHO * nb, a.partials + SLOT_RR2 * nb}, nb, sm, rhrr);
+    rho = rhrr[0];
     if (!a.true_residual && k > 1) {
-      residual = sqrt(reduce_partials(a.partials + SLOT_RR2 * nb, nb, sm)) / r0norm;
+      residual = sqrt(rhrr[1]) / r0norm;
       if (residual <= a.tol) { info = EGPU_HUTI_CONVERGENCE; iters = k - 1; break; }
       if (omega == 0.0) { info = EGPU_HUTI_BICGSTAB_OMEGA; iters = k - 1; break; }
       if (k > a.maxit) { info = EGPU_HUTI_MAXITER; iters = k - 1; break; }
@@ -1711,10 +1717,11 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
       store_partials(a, SLOT_RR, acc[1]);
     }
     if (!grid_barrier(a.bar, a.err, epoch)) return;
-    const double rv = reduce_partials(a.partials + SLOT_PQ * nb, nb, sm);
+    double rvrr[2];
+    reduce_partials_n<2>({a.partials + SLOT_PQ * nb, a.partials + SLOT_RR * nb}, nb, sm, rvrr);
+    const double rv = rvrr[0];
     if (a.true_residual && k > 1) {
-      const double rr = reduce_partials(a.partials + SLOT_RR * nb, nb, sm);
-      residual = sqrt(rr) / rhsnorm;
+      residual = sqrt(rvrr[1]) / rhsnorm;
       if (residual < a.tol) { info = EGPU_HUTI_CONVERGENCE; iters = k - 1; break; }
       if (omega == 0.0) { info = EGPU_HUTI_BICGSTAB_OMEGA; iters = k - 1; break; }
       if (k > a.maxit) { info = EGPU_HUTI_MAXITER; iters = k; break; }
@@ -1811,9 +1818,9 @@ __global__ void __launch_bounds__(EGPU_KBLOCK, 1) bicgstab_kernel(KArgs<VT> a) {
       store_partials(a, SLOT_TT, acc[1]);
     }
     if (!grid_barrier(a.bar, a.err, epoch)) return;
-    const double ss = reduce_partials(a.partials + SLOT_SS * nb, nb, sm);
-    const double ts = reduce_partials(a.partials + SLOT_TS * nb, nb, sm);
-    const double tt = reduce_partials(a.partials + SLOT_TT * nb, nb, sm);
+    double sts[3];
+    reduce_partials_n<3>({a.partials + SLOT_SS * nb, a.partials + SLOT_TS * nb, a.partials + SLOT_TT * nb}, nb, sm, sts);
+    const double ss = sts[0], ts = sts[1], tt = sts[2];
     if (sqrt(ss) < EGPU_HUTI_EPSILON) {
       const VT al = (VT)alpha;
       vec_loop<VT>(n, [&](int i, auto w) {

@@ -14,9 +14,9 @@ namespace egpu {
 // produce the value it waits for.
 constexpr int TRI_TS = 32;
 
-// occupancy-sized cooperative launch
+// occupancy-sized cooperative launch, of at most `most` blocks (0: no limit)
 template <typename K, typename Args>
-int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, size_t smem = 0) {
+int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, size_t smem = 0, int most = 0) {
   int bps = 0;
   if (smem > 48 * 1024)
     EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -29,12 +29,22 @@ int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, si
   if (args.nslices == 0) return EGPU_OK;  // the query above has loaded the kernel (krylov_load)
   bps = std::min(bps, 2048 / EGPU_KBLOCK);
   int grid = ctx->num_sms * bps;
+  if (most > 0) grid = std::min(grid, most);
   if (grid_out) *grid_out = grid;
   void *kargs[] = {&args};
   EGPU_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(EGPU_KBLOCK),
                                                  kargs, smem, ctx->stream));
   ctx->launches++;
   return EGPU_OK;
+}
+
+// Blocks of a solve without triangular solves: one for every SLICES_PER_BLOCK SELL slices.  A
+// small system's iteration is barriers and reductions, which cost less among fewer blocks; with
+// too few the slices of a block follow one another.  CG on hex 16^3 at 4, 8, 16, 32 and 64 slices
+// a block: 683, 658, 650, 658 and 853 us (all 148 blocks: 775); from 2368 slices on every SM has one.
+constexpr int SLICES_PER_BLOCK = 16;
+inline int krylov_blocks(int nslices) {
+  return std::max(1, (nslices + SLICES_PER_BLOCK - 1) / SLICES_PER_BLOCK);
 }
 
 // offs: 16-bit column offsets; form: a TriForm; smem: dynamic shared memory per block
