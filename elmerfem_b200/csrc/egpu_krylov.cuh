@@ -188,7 +188,7 @@ __device__ __forceinline__ VT ld_stream(const VT *p) {
   return __ldcs(p);
 }
 // Gathers of vectors written earlier in the same launch use plain cache-all loads: every
-// phase starts after grid_barrier, whose acquire fence discards stale L1 lines, and the
+// phase starts after grid_barrier, whose acquiring poll discards stale L1 lines, and the
 // stencil's reuse of x across neighbouring rows is then served from L1.
 template <typename VT>
 __device__ __forceinline__ VT ld_l2(const VT *p) {
@@ -200,6 +200,11 @@ __device__ __forceinline__ VT ld_l2(const VT *p) {
 // slice's entries column-major so each step of k is one coalesced 128-byte (FP32) or
 // 256-byte (FP64) warp load; each row sums in entry order.  Padding entries carry value 0
 // and a valid column.  epi(row, s0, s1) runs once per row on its own lane.
+//
+// The loops take U entries at a time, loads first; what is left over at the end of a row goes one
+// entry, two round trips, at a time, so U should divide the row: 9 for 27-point rows and 27-point
+// blocks (128^3 mixed CG's inner solves: 8 34.9 ms, 9 31.8 ms, 14 44.3, 27 37.0), else 5, the
+// tets' 15 entries (tet cube 40 mixed CG: 8 3.25 ms, 5 2.96 ms; hex at 5 35.2 ms).
 template <typename VT, int LPR, bool OFFS, bool TWO, typename F>
 __device__ __forceinline__ void spmv_phase(const KArgs<VT> &a, const VT *x0, const VT *x1, F &&epi) {
   const int lane = threadIdx.x & 31;
@@ -232,7 +237,7 @@ __device__ __forceinline__ void spmv_phase(const KArgs<VT> &a, const VT *x0, con
         for (int k0 = 0; k0 < w; k0 += 32) {
           const int kn = min(32, w - k0);
           const int offl = lane < kn ? (int)__ldg(co + k0 + lane) : 0;
-#pragma unroll 8
+#pragma unroll 9
           for (int k = 0; k < kn; ++k) {
             const VT v = ld_stream(a.svals + base + ((k0 + k) << 5));
             const int c = r + __shfl_sync(0xffffffffu, offl, k);
@@ -242,12 +247,22 @@ __device__ __forceinline__ void spmv_phase(const KArgs<VT> &a, const VT *x0, con
         }
       } else {
         const int16_t *co = a.scolsc + cp + lane;
-#pragma unroll 8
-        for (int k = 0; k < w; ++k) {
-          const VT v = ld_stream(a.svals + base + (k << 5));
-          const int c = r + (int)ld_stream(co + (k << 5));
-          s0 = row_madd(s0, v, ld_l2(x0 + c));
-          if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
+        if (w % 9) {
+#pragma unroll 5
+          for (int k = 0; k < w; ++k) {
+            const VT v = ld_stream(a.svals + base + (k << 5));
+            const int c = r + (int)ld_stream(co + (k << 5));
+            s0 = row_madd(s0, v, ld_l2(x0 + c));
+            if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
+          }
+        } else {
+#pragma unroll 9
+          for (int k = 0; k < w; ++k) {
+            const VT v = ld_stream(a.svals + base + (k << 5));
+            const int c = r + (int)ld_stream(co + (k << 5));
+            s0 = row_madd(s0, v, ld_l2(x0 + c));
+            if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
+          }
         }
       }
     } else {
