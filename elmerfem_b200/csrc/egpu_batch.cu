@@ -110,8 +110,10 @@ __device__ __forceinline__ SliceMeta batch_slice_meta(const BatchArgs &ba, const
   m.vals = d.svals + p;
   m.vbytes = (unsigned)(32 * w * (int)sizeof(float));
   if (d.scols16) {
-    m.cols = d.scols16 + p;
-    m.cbytes = (unsigned)(32 * w * (int)sizeof(int16_t));
+    if (__ldg(d.sell_cptr + sl) >= 0) {
+      m.cols = d.scols16 + p;
+      m.cbytes = (unsigned)(32 * w * (int)sizeof(int16_t));
+    }
   } else {
     m.cols = d.scols + p;
     m.cbytes = (unsigned)(32 * w * (int)sizeof(int));
@@ -158,20 +160,42 @@ __device__ __forceinline__ void batch_clear(const BatchArgs &a, int slot) {
     if (s % gridDim.x == (int)blockIdx.x) a.acc[slot * BATCH_MAX_SYS + s] = 0.0;
 }
 
-// SELL SpMV of one slice: lane's row sum of A x
-__device__ __forceinline__ float slice_spmv(const SysDesc &d, int slice, int lane, const float *x) {
-  const int r = (slice << 5) + lane;
-  const int w = __ldg(d.sell_w + slice);
-  const int base = __ldg(d.sell_ptr + slice) + lane;
+// A lane's sum of v * x over entries [k0, k1) of a SELL slice.  A slice whose rows share one
+// offset list reads it once (lane k holds offset k, broadcast by a shuffle), so its gathers wait
+// for no offset load.  SIDE < 0 / > 0: only entries below / above the diagonal (in a shared
+// slice every entry of the half's k range is).
+template <int SIDE>
+__device__ __forceinline__ float slice_sum(const SysDesc &d, const float *vals, int slice, int base, int r, int lane,
+                                           int k0, int k1, const float *x) {
   float s = 0.f;
+  const int cp = d.scols16 ? __ldg(d.sell_cptr + slice) : 0;
+  if (cp < 0) {
+    const float *vp = vals + base;
+    const int16_t *co = d.scolsc + (-cp - 1);
+    for (int b0 = k0; b0 < k1; b0 += 32) {
+      const int kn = min(32, k1 - b0);
+      const int offl = lane < kn ? (int)__ldg(co + b0 + lane) : 0;
 #pragma unroll 8
-  for (int k = 0; k < w; ++k) {
+      for (int k = 0; k < kn; ++k)
+        s = fmaf(__ldcs(vp + ((b0 + k) << 5)), __ldca(x + r + __shfl_sync(0xffffffffu, offl, k)), s);
+    }
+    return s;
+  }
+#pragma unroll 8
+  for (int k = k0; k < k1; ++k) {
     const int e = base + (k << 5);
-    const float v = __ldcs(d.svals + e);
+    const float v = __ldcs(vals + e);
     const int c = d.scols16 ? r + (int)__ldcs(d.scols16 + e) : __ldcs(d.scols + e);
-    s = fmaf(v, __ldca(x + c), s);
+    const bool take = SIDE == 0 || (SIDE < 0 ? c < r : c > r);
+    s = fmaf(take ? v : 0.f, __ldca(x + c), s);
   }
   return s;
+}
+
+// SELL SpMV of one slice: lane's row sum of A x
+__device__ __forceinline__ float slice_spmv(const SysDesc &d, int slice, int lane, const float *x) {
+  return slice_sum<0>(d, d.svals, slice, __ldg(d.sell_ptr + slice) + lane, (slice << 5) + lane, lane, 0,
+                      __ldg(d.sell_w + slice), x);
 }
 
 // Two slices of (possibly) different systems summed in one interleaved loop: a tet row has
@@ -226,7 +250,7 @@ __device__ __forceinline__ void batch_spmv1(const BatchArgs &ba, const BatchShar
     const int a = batch_locate(sh, q);
     if (lane == 0 && next.vbytes) {
       prefetch_l2_bulk(next.vals, next.vbytes);
-      prefetch_l2_bulk(next.cols, next.cbytes);
+      if (next.cbytes) prefetch_l2_bulk(next.cols, next.cbytes);
     }
     next = batch_slice_meta(ba, sh, q + 2 * nw, hi, run);
     const int s = sh.act[a];
@@ -251,11 +275,11 @@ __device__ __forceinline__ void batch_spmv2(const BatchArgs &ba, const BatchShar
     if (lane == 0) {
       if (n0.vbytes) {
         prefetch_l2_bulk(n0.vals, n0.vbytes);
-        prefetch_l2_bulk(n0.cols, n0.cbytes);
+        if (n0.cbytes) prefetch_l2_bulk(n0.cols, n0.cbytes);
       }
       if (n1.vbytes) {
         prefetch_l2_bulk(n1.vals, n1.vbytes);
-        prefetch_l2_bulk(n1.cols, n1.cbytes);
+        if (n1.cbytes) prefetch_l2_bulk(n1.cols, n1.cbytes);
       }
     }
     n0 = batch_slice_meta(ba, sh, q0 + 2 * step, hi, run);
@@ -480,6 +504,29 @@ __device__ __forceinline__ void batch_tri_any(const BatchArgs &a, const BatchSha
 // ------------------------------------------------------------------------------------
 // the kernel
 
+// the factor entries (and offsets, where the slice stores its own) of slice rank q's half
+template <bool UPPER>
+__device__ __forceinline__ SliceMeta batch_sweep_meta(const BatchArgs &ba, const BatchShared &sh, int q, int hi) {
+  SliceMeta m{nullptr, nullptr, 0u, 0u};
+  if (q >= hi) return m;
+  const int a = batch_locate(sh, q);
+  const int s = sh.act[a];
+  if (sh.status[s] != ST_RUN) return m;
+  const SysDesc &d = ba.sys[s];
+  const int sl = q - sh.pre[a];
+  const int p = __ldg(d.sell_ptr + sl), w = __ldg(d.sell_w + sl);
+  const int2 rg = __ldg(d.swr + sl);
+  const int k0 = UPPER ? rg.y : 0, k1 = UPPER ? w : rg.x;
+  if (k1 <= k0) return m;
+  m.vals = d.isvals + p + 32 * k0;
+  m.vbytes = (unsigned)(32 * (k1 - k0) * (int)sizeof(float));
+  if (d.scols16 && __ldg(d.sell_cptr + sl) >= 0) {
+    m.cols = d.scols16 + p + 32 * k0;
+    m.cbytes = (unsigned)(32 * (k1 - k0) * (int)sizeof(int16_t));
+  }
+  return m;
+}
+
 // One Jacobi sweep over the running systems' ILU0 factors (see sweep_phase in
 // egpu_krylov.cuh): a warp per slice, lane = row, the entries with col < row (LOWER) or
 // col > row (UPPER) of the slice's k range.  zin(s): the vector system s multiplies;
@@ -489,9 +536,14 @@ __device__ __forceinline__ void batch_sweep(const BatchArgs &ba, const BatchShar
   const int total = sh.total, nb = gridDim.x;
   const int lo = (int)((long long)total * blockIdx.x / nb), hi = (int)((long long)total * (blockIdx.x + 1) / nb);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+  // lane 0 prefetches the factor entries of the slice the warp takes next into L2 (as batch_spmv1)
+  SliceMeta next = batch_sweep_meta<UPPER>(ba, sh, lo + warp + nw, hi);
   for (int q = lo + warp; q < hi; q += nw) {
     const int a = batch_locate(sh, q);
     const int s = sh.act[a];
+    if (lane == 0 && next.vbytes) prefetch_l2_bulk(next.vals, next.vbytes);
+    if (lane == 0 && next.cbytes) prefetch_l2_bulk(next.cols, next.cbytes);
+    next = batch_sweep_meta<UPPER>(ba, sh, q + 2 * nw, hi);
     if (sh.status[s] != ST_RUN) continue;
     const SysDesc &d = ba.sys[s];
     const int slice = q - sh.pre[a];
@@ -499,17 +551,8 @@ __device__ __forceinline__ void batch_sweep(const BatchArgs &ba, const BatchShar
     const int w = __ldg(d.sell_w + slice);
     const int2 rg = __ldg(d.swr + slice);
     const int k0 = UPPER ? rg.y : 0, k1 = UPPER ? w : rg.x;
-    const int base = __ldg(d.sell_ptr + slice) + lane;
-    const float *z = zin(s);
-    float sum = 0.f;
-#pragma unroll 4
-    for (int k = k0; k < k1; ++k) {
-      const int e = base + (k << 5);
-      const int c = d.scols16 ? r + (int)__ldcs(d.scols16 + e) : __ldcs(d.scols + e);
-      const float v = __ldcs(d.isvals + e);
-      const bool take = UPPER ? c > r : c < r;
-      sum = fmaf(take ? v : 0.f, __ldca(z + c), sum);
-    }
+    const float sum = slice_sum<(UPPER ? 1 : -1)>(d, d.isvals, slice, __ldg(d.sell_ptr + slice) + lane, r, lane, k0,
+                                                  k1, zin(s));
     if (r < d.n) epi(s, r, sum);
   }
 }
@@ -1144,34 +1187,42 @@ struct TeamArgs {
 };
 
 // barrier of one team (T CTAs; a block barrier when T = 1), bounded like grid_barrier.  The
-// error word is read once, by thread 0, and broadcast, so the whole block takes the same way out.
+// error word is read by thread 0, and broadcast, so the whole block takes the same way out: with
+// several CTAs while the counter is polled, with one CTA at every TEAM_ERR_EVERY-th barrier only
+// (read at each, its L2 round trip was most of a small system's barrier).
+constexpr unsigned TEAM_ERR_EVERY = 32;
 __device__ __forceinline__ bool team_sync(unsigned int *cnt, int team, unsigned int &epoch, int *err) {
-  __shared__ int ok_s;
+  epoch += 1;
+  if (team == 1) {
+    if (epoch % TEAM_ERR_EVERY) {
+      __syncthreads();
+      return true;
+    }
+    return __syncthreads_or(threadIdx.x == 0 && *(volatile int *)err != 0) == 0;
+  }
   __syncthreads();
-  if (team > 1) {
-    epoch += 1;
-    if (threadIdx.x == 0) {
-      const unsigned int target = epoch * (unsigned int)team;
-      red_release_add_u32(cnt, 1u);
-      if (ld_acquire_u32(cnt) < target) {
-        const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(err);
-        unsigned int spins = 0;
-        while (ld_acquire_u32(cnt) < target) {
-          if ((++spins & 63u) == 0) {
-            if (*(volatile int *)err) break;
-            if (egpu_globaltimer() - t0 > lim) {
-              atomicCAS(err, 0, (int)EGPU_ERR_TIMEOUT);
-              break;
-            }
+  int bad = 0;
+  if (threadIdx.x == 0) {
+    const unsigned int target = epoch * (unsigned int)team;
+    red_release_add_u32(cnt, 1u);
+    bad = *(volatile int *)err;
+    unsigned int c = ld_acquire_u32(cnt);
+    if (c < target) {
+      const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(err);
+      unsigned int spins = 0;
+      while ((c = ld_acquire_u32(cnt)) < target) {
+        if ((++spins & 63u) == 0) {
+          if (*(volatile int *)err) break;
+          if (egpu_globaltimer() - t0 > lim) {
+            atomicCAS(err, 0, (int)EGPU_ERR_TIMEOUT);
+            break;
           }
         }
       }
-      __threadfence();
+      if (c < target) bad = 1;
     }
   }
-  if (threadIdx.x == 0) ok_s = *(volatile int *)err == 0;
-  __syncthreads();
-  return ok_s != 0;
+  return __syncthreads_or(bad) == 0;
 }
 
 // NV team-wide sums: the block's sums of v, one partial per member in slots [slot, slot + NV),
@@ -1203,6 +1254,20 @@ __device__ __forceinline__ void team_vec(int r0, int r1, F &&f) {
 #pragma unroll 4
   for (int q = q0 + (int)threadIdx.x; q < q1; q += blockDim.x) f(q << 2, VW<4>{});
   for (int i = (q1 << 2) + (int)threadIdx.x; i < r1; i += blockDim.x) f(i, VW<1>{});
+}
+
+// A lane's row sum, U entries at a time.  The unrolling should divide the row: what is left over
+// after the last whole chunk goes one entry, two round trips, at a time.  5 for the tets' 15
+// entries, 9 for 27-point rows (96 tet systems: 16 82 ms, 15 54 ms, 5 52 ms).
+template <int U>
+__device__ __forceinline__ float team_row(const TeamSys &S, const float *P, int r, int base, int w) {
+  float t = 0.f;
+#pragma unroll U
+  for (int kk = 0; kk < w; ++kk) {
+    const int e = base + (kk << 5);
+    t = fmaf(__ldcs(S.svals32 + e), __ldca(P + r + (int)__ldcs(S.scols16 + e)), t);
+  }
+  return t;
 }
 
 // one member's whole solve of system S; false on a recorded error
@@ -1309,18 +1374,16 @@ __device__ bool team_solve(const TeamArgs &a, const TeamSys &S, int rank, TeamOu
           if (S.scols16) prefetch_l2_bulk(S.scols16 + p2, (unsigned)(64 * w2));
         }
         float t = 0.f;
-        if (S.scols16) {
-#pragma unroll 16
-          for (int kk = 0; kk < w; ++kk) {
-            const int e = base + (kk << 5);
-            t = fmaf(__ldcs(S.svals32 + e), __ldca(P + r + (int)__ldcs(S.scols16 + e)), t);
-          }
-        } else {
+        if (!S.scols16) {
 #pragma unroll 8
           for (int kk = 0; kk < w; ++kk) {
             const int e = base + (kk << 5);
             t = fmaf(__ldcs(S.svals32 + e), __ldca(P + __ldcs(S.scols + e)), t);
           }
+        } else if (w % 9) {
+          t = team_row<5>(S, P, r, base, w);
+        } else {
+          t = team_row<9>(S, P, r, base, w);
         }
         if (r < n) {
           Q[r] = t;
@@ -1544,6 +1607,8 @@ static int batch_prepare(egpu_batch *B, int slot, const double *b_dev) {
   d.sell_ptr = A->sell_ptr.p;
   d.sell_w = A->sell_w.p;
   d.scols16 = A->sell_c16.p;
+  d.sell_cptr = A->sell_cptr.p;
+  d.scolsc = A->sell_csc.p;
   d.scols = A->sell_cols.p;
   d.svals = A->sell_vals32.p;
   d.dvals = A->work32.p + 13 * ldw32;

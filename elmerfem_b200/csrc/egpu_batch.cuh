@@ -36,6 +36,9 @@ struct SysDesc {
   const int *sell_ptr, *sell_w;
   const int16_t *scols16;  // col - row
   const int *scols;        // absolute column (when scols16 is null)
+  // offsets of scols16 with one list for a slice whose rows share it (see egpu_mat::sell_cptr)
+  const int *sell_cptr;
+  const int16_t *scolsc;
   const float *svals, *dvals, *ilu;
   const int *rows, *cols, *diag, *lower_order, *upper_order;
   const int *lo_ptr, *lo_cols, *up_ptr, *up_cols;   // ILU0 factors packed in solve order
