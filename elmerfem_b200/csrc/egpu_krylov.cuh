@@ -588,11 +588,13 @@ __device__ __forceinline__ void upper_solve_blk(const KArgs<VT> &a, const VT *y,
 // barrier among the first nt threads of the block (named barrier 1; nt a multiple of 32)
 __device__ __forceinline__ void cta_bar(int nt) { asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory"); }
 
-// mbarriers of the stages (copied; read), then the number of levels staged so far in this launch
+// mbarriers of the stages (copied; read), then the number of levels staged so far in this launch,
+// then a word set when a wait for a stage ran out
 constexpr int RANGE_COUNT_AT = 16 * plan::RANGE_STAGES;
+constexpr int RANGE_BROKEN_AT = RANGE_COUNT_AT + 4;
 constexpr int RANGE_FETCH = 8;   // warps fetching external values
 constexpr int RANGE_AHEAD = 16;  // levels prefetched into L2
-constexpr int RANGE_HEAD = 16 * ((RANGE_COUNT_AT + 4 + 15) / 16);
+constexpr int RANGE_HEAD = 16 * ((RANGE_BROKEN_AT + 4 + 15) / 16);
 // stage: bytes of the largest level record
 template <typename VT>
 __host__ __device__ constexpr size_t range_smem_bytes(int rows, int ext, int stage) {
@@ -665,6 +667,7 @@ struct RangeRun {
   unsigned sx, srhs, stage, bar;
   VT *x;
   int *err;
+  volatile int *broken;  // shared memory: a wait for a stage ran out in this launch
   int rows, stage_bytes, lg, nt;
   unsigned first;  // levels staged before this triangle (stage and parity go on)
 };
@@ -680,6 +683,14 @@ __device__ __forceinline__ void range_arrive(int id, int nt) { asm volatile("bar
 // cycles a level with one set, which read its next entries in between).  The barrier that starts
 // level m: its set waits, the other arrives when level m - 1 is stored.
 // The next warp stages level records, RANGE_STAGES ahead; the rest fetch external values.
+//
+// An error (another block's, or an external value that never comes) ends the waits for values
+// only.  The waits for stages go on until the copy is there, so the sets never run ahead of the
+// copies: a set more than RANGE_STAGES levels ahead would take the barrier's other phase, which
+// has the same parity, for its own, and read a record while it is overwritten.  A wait for a
+// stage that does run out ends every read of stages by that thread, and the block solves no
+// further triangle in this launch (R.broken): its barriers' phases no longer match the levels.
+// All copies have landed when this returns.
 // Returns the levels staged.
 template <typename VT, int K>
 __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT> R) {
@@ -694,15 +705,21 @@ __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT>
     unsigned xa[K];  // addresses of the entries' values
     int row = -1;
     unsigned dst = 0;
+    bool lost = false;  // a stage did not arrive in time: none is read any more
     // the entries of level m, from its stage into registers
     auto load = [&](int m) {
       const unsigned q = R.first + m, st = q % S, bar = R.bar + 8 * st, ph = (q / S) & 1u;
       row = -1;
-      bool here = mbar_try(bar, ph);
-      if (!here) {  // bounded; once an error is recorded, no level waits again or is solved
-        unsigned long long t0 = 0;
-        for (unsigned int spin = 64; !(here = mbar_try(bar, ph)); spin += 64)
-          if (range_wait_over(spin, t0, R.err)) break;
+      bool here = !lost && mbar_try(bar, ph);
+      if (!here && !lost) {
+        const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(R.err);
+        while (!(here = mbar_try(bar, ph)))
+          if (egpu_globaltimer() - t0 > lim) {
+            atomicCAS(R.err, 0, (int)EGPU_ERR_TIMEOUT);
+            *R.broken = 1;
+            lost = true;
+            break;
+          }
       }
       const unsigned rec = R.stage + st * (unsigned)R.stage_bytes;
       int s0 = 0, w = 0;
@@ -768,19 +785,23 @@ __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT>
     }
   } else if ((int)threadIdx.x < nbar + 32) {
     // One thread issues.  It reuses a stage when all warps of the set have read it and the copy
-    // before is complete (it is, except after an error, when the solving threads stop waiting),
-    // so at most RANGE_STAGES are in flight, and after an error it sees those end too.
+    // before is complete (it is, except where a thread gave up its wait for it), so at most
+    // RANGE_STAGES are in flight, and it sees those end before it returns: a copy must not land in
+    // the shared memory of a block that has exited.  That last wait is bounded by EGPU_WAIT_NS and
+    // not by the context's limit, which may be shorter than a copy.
     if ((int)threadIdx.x == nbar) {
-      auto wait = [&](unsigned bar, unsigned ph) {
+      auto wait = [&](unsigned bar, unsigned ph, unsigned long long lim) {
         if (mbar_try(bar, ph)) return true;
-        const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(R.err);
+        const unsigned long long t0 = egpu_globaltimer();
         while (!mbar_try(bar, ph))
           if (egpu_globaltimer() - t0 > lim) {
-            atomicExch(R.err, (int)EGPU_ERR_TIMEOUT);
+            atomicCAS(R.err, 0, (int)EGPU_ERR_TIMEOUT);
+            *R.broken = 1;
             return false;
           }
         return true;
       };
+      const unsigned long long lim = egpu_wait_limit(R.err);
       auto bar = [&](unsigned q) { return R.bar + 8 * (q % S); };
       auto phase = [&](unsigned q) { return (q / S) & 1u; };
       int l = 0;
@@ -788,7 +809,7 @@ __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT>
       for (; l < nl; ++l) {
         const unsigned q = R.first + l;
         const long long o1 = __ldg(T.offset + l0 + l + 1);
-        if (q >= S && (!wait(bar(q) + 8 * S, phase(q - S)) || !wait(bar(q), phase(q - S)))) break;
+        if (q >= S && (!wait(bar(q) + 8 * S, phase(q - S), lim) || !wait(bar(q), phase(q - S), lim))) break;
         bulk_load(R.stage + (q % S) * (unsigned)R.stage_bytes, T.rec + o0, (unsigned)(o1 - o0), bar(q));
         o0 = o1;
         // the level RANGE_AHEAD later into L2: the stages alone cover an L2 hit, not HBM
@@ -797,8 +818,7 @@ __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT>
           prefetch_l2_bulk(T.rec + p0, (unsigned)(p1 - p0));
         }
       }
-      if (*(volatile int *)R.err)
-        for (int h = max(0, l - S); h < l; ++h) wait(bar(R.first + h), phase(R.first + h));
+      for (int h = max(0, l - S); h < l; ++h) wait(bar(R.first + h), phase(R.first + h), EGPU_WAIT_NS);
     }
   } else {
     // External values, in the order of their first use, 32 a warp at a time, by at most
@@ -834,7 +854,10 @@ __device__ __forceinline__ void range_init(int nt) {
   extern __shared__ __align__(16) unsigned char egpu_dsm[];
   if (threadIdx.x < 2 * plan::RANGE_STAGES)
     mbar_init(smem_u32(egpu_dsm) + 8 * threadIdx.x, threadIdx.x < plan::RANGE_STAGES ? 1u : (unsigned)nt / 32);
-  if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned *>(egpu_dsm + RANGE_COUNT_AT) = 0u;
+  if (threadIdx.x == 0) {
+    *reinterpret_cast<volatile unsigned *>(egpu_dsm + RANGE_COUNT_AT) = 0u;
+    *reinterpret_cast<volatile int *>(egpu_dsm + RANGE_BROKEN_AT) = 0;
+  }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
 }
@@ -870,10 +893,12 @@ __device__ __forceinline__ void range_ilu(const KArgs<VT> &a, VT *y, VT *z, RHS 
         srhs[__ldg(a.rlo.slot + r)] = v;
       }
   }
-  __syncthreads();
+  // read before the barrier: all threads of the block take the same way
+  volatile int *broken = reinterpret_cast<volatile int *>(egpu_dsm + RANGE_BROKEN_AT);
+  const bool lower = __syncthreads_or(*broken) == 0;
   RangeRun<VT> run{smem_u32(sx), smem_u32(srhs), smem_u32(stage), smem_u32(egpu_dsm), y,       a.err,
-                   a.rg_rows,    a.rg_stage,     a.rg_lg,         a.rg_nt,            *count};
-  if (cnt > 0) run.first += (unsigned)range_triangle<VT, K>(a.rlo, run);
+                   broken,       a.rg_rows,      a.rg_stage,      a.rg_lg,            a.rg_nt, *count};
+  if (cnt > 0 && lower) run.first += (unsigned)range_triangle<VT, K>(a.rlo, run);
   __syncthreads();
   for (int i = threadIdx.x; i < a.rg_ext; i += blockDim.x) sx[a.rg_rows + i] = Sentinel<VT>::value();
   // y times the inverse of the node block's upper triangle (inverted diagonal included)
@@ -893,9 +918,9 @@ __device__ __forceinline__ void range_ilu(const KArgs<VT> &a, VT *y, VT *z, RHS 
       }
     }
   }
-  __syncthreads();
+  const bool upper = __syncthreads_or(*broken) == 0;
   run.x = z;
-  if (cnt > 0) run.first += (unsigned)range_triangle<VT, K>(a.rup, run);
+  if (cnt > 0 && upper) run.first += (unsigned)range_triangle<VT, K>(a.rup, run);
   __syncthreads();
   if (threadIdx.x == 0) *count = run.first;
   for (int i = threadIdx.x; i < cnt; i += blockDim.x) out(base + i, sx[__ldg(a.rup.slot + base + i)]);
