@@ -429,7 +429,7 @@ __device__ __forceinline__ void batch_tri_group(const BatchArgs &a, const BatchS
       beg = __ldg(ptr + pos);
       end = __ldg(ptr + pos + 1);
       if (row < 0 || row >= d.n || end < beg) {
-        if (sl == 0) atomicExch(a.err, (int)EGPU_ERR_ARG);
+        if (sl == 0) egpu_record(a.err, (int)EGPU_ERR_ARG);
         valid = false;
         row = -1;
       } else {
@@ -440,7 +440,7 @@ __device__ __forceinline__ void batch_tri_group(const BatchArgs &a, const BatchS
             c[u] = __ldg(cols + e);
             v[u] = __ldg(vals + e);
             if (c[u] < 0 || c[u] >= d.n) {
-              atomicExch(a.err, (int)EGPU_ERR_ARG);
+              egpu_record(a.err, (int)EGPU_ERR_ARG);
               c[u] = -1;
             }
           }
@@ -466,7 +466,7 @@ __device__ __forceinline__ void batch_tri_group(const BatchArgs &a, const BatchS
       for (int e = beg + E * TS + sl; e < end; e += TS) {
         const int cc = __ldg(cols + e);
         if (cc < 0 || cc >= d.n) {
-          atomicExch(a.err, (int)EGPU_ERR_ARG);
+          egpu_record(a.err, (int)EGPU_ERR_ARG);
           continue;
         }
         acc += __ldg(vals + e) * Sentinel<float>::wait(x + cc, a.err);
@@ -1198,23 +1198,23 @@ __device__ __forceinline__ bool team_sync(unsigned int *cnt, int team, unsigned 
       __syncthreads();
       return true;
     }
-    return __syncthreads_or(threadIdx.x == 0 && *(volatile int *)err != 0) == 0;
+    return __syncthreads_or(threadIdx.x == 0 && egpu_error(err) != 0) == 0;
   }
   __syncthreads();
   int bad = 0;
   if (threadIdx.x == 0) {
     const unsigned int target = epoch * (unsigned int)team;
     red_release_add_u32(cnt, 1u);
-    bad = *(volatile int *)err;
+    bad = egpu_error(err);
     unsigned int c = ld_acquire_u32(cnt);
     if (c < target) {
       const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(err);
       unsigned int spins = 0;
       while ((c = ld_acquire_u32(cnt)) < target) {
         if ((++spins & 63u) == 0) {
-          if (*(volatile int *)err) break;
+          if (egpu_error(err)) break;
           if (egpu_globaltimer() - t0 > lim) {
-            atomicCAS(err, 0, (int)EGPU_ERR_TIMEOUT);
+            egpu_record(err, (int)EGPU_ERR_TIMEOUT);
             break;
           }
         }
@@ -1449,7 +1449,7 @@ __global__ void __launch_bounds__(TEAM_BLOCK, TEAM_PER_SM) k_batch_team(TeamArgs
     __syncthreads();
     if (threadIdx.x == 0) {
       egpu_poll_abort(a.err);
-      task = *(volatile int *)a.err ? a.ntasks : (int)atomicAdd(a.next, 1u);
+      task = egpu_error(a.err) ? a.ntasks : (int)atomicAdd(a.next, 1u);
     }
     __syncthreads();
     const int t = task;

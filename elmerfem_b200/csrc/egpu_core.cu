@@ -273,12 +273,12 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
   for (int s = gw; s < n; s += nw) {
     const int i = order[s];
     if (i < 0 || i >= n) {
-      if (lane == 0) atomicExch(err, (int)EGPU_ERR_ARG);
+      if (lane == 0) egpu_record(err, (int)EGPU_ERR_ARG);
       return;
     }
     const int beg = rows[i], len = rows[i + 1] - beg, nl = diag[i] - beg;
     if ((MAXROW > 0 && len > MAXROW) || nl < 0 || nl > len) {
-      if (lane == 0) atomicExch(err, (int)EGPU_ERR_ARG);
+      if (lane == 0) egpu_record(err, (int)EGPU_ERR_ARG);
       return;
     }
     double *S = MAXROW > 0 ? S_all[wib] : ilu + beg;
@@ -311,10 +311,10 @@ __global__ void __launch_bounds__(256) k_ilu0_factor(int n, const int *__restric
         if (t0 == 0) t0 = egpu_globaltimer();
         if ((++spin & 31u) == 0) {
           int stop = 0;
-          if (lane == 0) stop = egpu_globaltimer() - t0 > egpu_wait_limit(err) ? 1 : (*(volatile int *)err ? 2 : 0);
+          if (lane == 0) stop = egpu_globaltimer() - t0 > egpu_wait_limit(err) ? 1 : (egpu_error(err) ? 2 : 0);
           stop = __shfl_sync(0xffffffffu, stop, 0);
           if (stop) {
-            if (stop == 1 && lane == 0) atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+            if (stop == 1 && lane == 0) egpu_record(err, (int)EGPU_ERR_TIMEOUT);
             return;
           }
         }

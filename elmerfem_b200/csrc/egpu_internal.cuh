@@ -25,11 +25,12 @@
 #define EGPU_WAIT_NS 2000000000ull
 
 // The context's device control block is its sync buffer of EGPU_SYNC_WORDS 32-bit words:
-// word 0 the grid-barrier counter, word 1 the error word every kernel reports to, words
-// 2..63 per-solve scratch (cleared before each solve), and from EGPU_CTL_WORD on the words
-// that persist across solves: the wait bound in ns (u64, 0 = EGPU_WAIT_NS) and the device
-// address of the host-mapped abort word (u64, 0 = none).  Kernels receive a pointer to the
-// error word and find the control words at a fixed distance from it.
+// word 0 the grid-barrier counter, word 1 the error word every kernel reports to (kernels reach
+// the two as one 64-bit word: grid_barrier, egpu_error, egpu_record), words 2..63 per-solve
+// scratch (cleared before each solve), and from EGPU_CTL_WORD on the words that persist across
+// solves: the wait bound in ns (u64, 0 = EGPU_WAIT_NS) and the device address of the host-mapped
+// abort word (u64, 0 = none).  Kernels receive a pointer to the error word and find the control
+// words at a fixed distance from it.
 #define EGPU_SYNC_WORDS 128
 #define EGPU_CTL_WORD 64
 #define EGPU_SELFTEST_WORD 96
@@ -316,6 +317,14 @@ __device__ __forceinline__ void st_release_s32(int *p, int v) {
 __device__ __forceinline__ void red_release_add_u32(unsigned int *p, unsigned int v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ void red_release_add_u64(void *p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const void *p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const void *p) {
   unsigned long long v;
@@ -341,13 +350,31 @@ __device__ __forceinline__ unsigned long long egpu_wait_limit(const int *err) {
   return v ? v : EGPU_WAIT_NS;
 }
 
+// The error word and the barrier counter before it, as the one 64-bit word that grid_barrier
+// polls.  Every access of a kernel that uses the barrier has this width: two accesses that overlap
+// in part only are a data race without any guarantee, also where both are atomic.
+__device__ __forceinline__ unsigned long long *egpu_ctl_pair(const int *err) {
+  return (unsigned long long *)(err - 1);
+}
+// the recorded error, 0: none
+__device__ __forceinline__ int egpu_error(const int *err) { return (int)(ld_relaxed_u64(egpu_ctl_pair(err)) >> 32); }
+// records an error unless one is recorded already; the counter beside it is kept
+static __device__ __noinline__ void egpu_record(int *err, int code) {
+  unsigned long long *w = egpu_ctl_pair(err), old = ld_relaxed_u64(w);
+  while ((old >> 32) == 0) {
+    const unsigned long long seen = atomicCAS(w, old, (old & 0xffffffffull) | ((unsigned long long)(unsigned int)code << 32));
+    if (seen == old) break;
+    old = seen;  // an arrival (finitely many) or another error
+  }
+}
+
 // Reads the context's host-mapped abort word (one load over the host link) and, when the host
 // has raised it, records EGPU_ERR_ABORT unless another error is already recorded; every
 // block then leaves at its next grid barrier or bounded wait.
 __device__ __forceinline__ void egpu_poll_abort(int *err) {
   const unsigned long long a =
       *(const volatile unsigned long long *)((const unsigned int *)err + (EGPU_CTL_WORD + 1));
-  if (a && *(const volatile int *)a) atomicCAS(err, 0, (int)EGPU_ERR_ABORT);
+  if (a && *(const volatile int *)a) egpu_record(err, (int)EGPU_ERR_ABORT);
 }
 
 // value type traits for the sync-free solves
@@ -369,10 +396,10 @@ struct Sentinel<double> {
       if (v != EGPU_SENTINEL64) break;
       if ((spin & 31u) == 0) {
         if (egpu_globaltimer() - t0 > lim) {
-          atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+          egpu_record(err, (int)EGPU_ERR_TIMEOUT);
           break;
         }
-        if (*(volatile int *)err) break;
+        if (egpu_error(err)) break;
       }
     }
     return __longlong_as_double((long long)v);
@@ -398,10 +425,10 @@ struct Sentinel<float> {
       if (v != EGPU_SENTINEL32) break;
       if ((spin & 31u) == 0) {
         if (egpu_globaltimer() - t0 > lim) {
-          atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+          egpu_record(err, (int)EGPU_ERR_TIMEOUT);
           break;
         }
-        if (*(volatile int *)err) break;
+        if (egpu_error(err)) break;
       }
     }
     return __uint_as_float(v);
@@ -420,15 +447,12 @@ struct Sentinel<float> {
 // solves, the ILU factorisation) doubled the set-up time of a large solve.  Returns false
 // when the kernel must unwind (error flag set by anyone).
 #define EGPU_ABORT_POLL 256u
-// The counter and the error word are neighbours (words 0 and 1 of the control block), so one
-// 64-bit acquire load polls both; its result reaches the block through the closing barrier
-// (a separate read of the error word by every thread, and a fence after the poll, cost about
-// 0.6 us of the barrier).
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const void *p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
+// The counter and the error word are the halves of one 64-bit word (egpu_ctl_pair; count + 1 is
+// err).  A block arrives with a 64-bit release addition and polls with a 64-bit acquire load, the
+// same width, so that the release and the acquire order the phases before and after the barrier;
+// the load brings the error word along, and its result reaches the block through the closing
+// barrier (a separate read of the error word by every thread, and a fence after the poll, cost
+// about 0.6 us of the barrier).
 #ifdef EGPU_BARRIER_CALL
 static __device__ __noinline__
 #else
@@ -441,7 +465,7 @@ bool grid_barrier(unsigned int *count, int *err, unsigned int &epoch) {
   if (threadIdx.x == 0) {
     if (blockIdx.x == 0 && (epoch % EGPU_ABORT_POLL) == 0) egpu_poll_abort(err);
     const unsigned int target = epoch * gridDim.x;
-    red_release_add_u32(count, 1u);
+    red_release_add_u64(count, 1ull);
     unsigned long long w = ld_acquire_u64(count);
     if ((unsigned int)w < target) {
       const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(err);
@@ -450,9 +474,9 @@ bool grid_barrier(unsigned int *count, int *err, unsigned int &epoch) {
         if ((++spins & 63u) == 0) {
           // one block polls during long waits (block 0 may be the one still working)
           if ((spins & 1023u) == 0 && blockIdx.x == (gridDim.x > 1 ? 1u : 0u)) egpu_poll_abort(err);
-          if (*(volatile int *)err) break;
+          if (egpu_error(err)) break;
           if (egpu_globaltimer() - t0 > lim) {
-            atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+            egpu_record(err, (int)EGPU_ERR_TIMEOUT);
             break;
           }
         }

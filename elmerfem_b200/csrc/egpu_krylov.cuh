@@ -314,10 +314,10 @@ __device__ __forceinline__ void warp_wait_all(VT (&xv)[E], const int (&c)[E], co
     if ((spin & 31u) == 0) {
       int stop = 0;
       if ((threadIdx.x & 31) == 0)
-        stop = egpu_globaltimer() - t0 > egpu_wait_limit(err) ? 1 : (*(volatile int *)err ? 2 : 0);
+        stop = egpu_globaltimer() - t0 > egpu_wait_limit(err) ? 1 : (egpu_error(err) ? 2 : 0);
       stop = __shfl_sync(0xffffffffu, stop, 0);
       if (stop) {
-        if (stop == 1 && (threadIdx.x & 31) == 0) atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+        if (stop == 1 && (threadIdx.x & 31) == 0) egpu_record(err, (int)EGPU_ERR_TIMEOUT);
         return;
       }
     }
@@ -344,7 +344,7 @@ __device__ __forceinline__ void tri_fetch(TriRow<VT> &t, int s, const int *order
   t.c0 = t.c1 = -1;
   t.v0 = t.v1 = 0;
   if (t.row < 0 || t.row >= n || t.end < t.beg) {
-    if (lane == 0) atomicExch(err, (int)EGPU_ERR_ARG);
+    if (lane == 0) egpu_record(err, (int)EGPU_ERR_ARG);
     t.row = -1;
     t.end = t.beg;
     return;
@@ -358,7 +358,7 @@ __device__ __forceinline__ void tri_fetch(TriRow<VT> &t, int s, const int *order
     t.c1 = __ldg(cols + t.beg + 32 + lane);
   }
   if (t.c0 >= n || t.c1 >= n) {
-    atomicExch(err, (int)EGPU_ERR_ARG);
+    egpu_record(err, (int)EGPU_ERR_ARG);
     if (t.c0 >= n) t.c0 = -1;
     if (t.c1 >= n) t.c1 = -1;
   }
@@ -440,7 +440,7 @@ __device__ __forceinline__ void blk_dot(VT (&acc)[TRI_BS_MAX], const int (&p)[TR
     int k;
     c[u] = blk_ext<LOWER>(p, bs, e, k) ? __ldg(cols + e) : -1;
     if (c[u] >= n) {
-      atomicExch(err, (int)EGPU_ERR_ARG);
+      egpu_record(err, (int)EGPU_ERR_ARG);
       c[u] = -1;
     }
   }
@@ -463,7 +463,7 @@ __device__ __forceinline__ void blk_dot(VT (&acc)[TRI_BS_MAX], const int (&p)[TR
     if (!blk_ext<LOWER>(p, bs, e, k)) continue;
     const int cc = __ldg(cols + e);
     if (cc < 0 || cc >= n) {
-      atomicExch(err, (int)EGPU_ERR_ARG);
+      egpu_record(err, (int)EGPU_ERR_ARG);
       continue;
     }
     blk_add(acc, k, __ldg(vals + e) * Sentinel<VT>::wait(x + cc, err));
@@ -485,7 +485,7 @@ __device__ __forceinline__ bool blk_fetch(int q0, int bs, const int *order, cons
 #pragma unroll
   for (int q = 0; q < TRI_BS_MAX; ++q)
     if (q < bs) ok = ok && p[q + 1] - p[q] >= q;
-  if (!ok && (threadIdx.x & 31) == 0) atomicExch(err, (int)EGPU_ERR_ARG);
+  if (!ok && (threadIdx.x & 31) == 0) egpu_record(err, (int)EGPU_ERR_ARG);
   return ok;
 }
 
@@ -628,11 +628,11 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigne
 // every 64th round of a wait: true when it has to end (limit passed, or an error recorded)
 __device__ __forceinline__ bool range_wait_over(unsigned int spin, unsigned long long &t0, int *err) {
   if (spin & 63u) return false;
-  if (*(volatile int *)err) return true;
+  if (egpu_error(err)) return true;
   const unsigned long long t = egpu_globaltimer();
   if (t0 == 0) t0 = t;
   if (t - t0 > egpu_wait_limit(err)) {
-    atomicExch(err, (int)EGPU_ERR_TIMEOUT);
+    egpu_record(err, (int)EGPU_ERR_TIMEOUT);
     return true;
   }
   return false;
@@ -715,7 +715,7 @@ __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT>
         const unsigned long long t0 = egpu_globaltimer(), lim = egpu_wait_limit(R.err);
         while (!(here = mbar_try(bar, ph)))
           if (egpu_globaltimer() - t0 > lim) {
-            atomicCAS(R.err, 0, (int)EGPU_ERR_TIMEOUT);
+            egpu_record(R.err, (int)EGPU_ERR_TIMEOUT);
             *R.broken = 1;
             lost = true;
             break;
@@ -795,7 +795,7 @@ __device__ __noinline__ int range_triangle(const RangeTri &T, const RangeRun<VT>
         const unsigned long long t0 = egpu_globaltimer();
         while (!mbar_try(bar, ph))
           if (egpu_globaltimer() - t0 > lim) {
-            atomicCAS(R.err, 0, (int)EGPU_ERR_TIMEOUT);
+            egpu_record(R.err, (int)EGPU_ERR_TIMEOUT);
             *R.broken = 1;
             return false;
           }

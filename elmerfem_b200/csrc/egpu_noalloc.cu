@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) k_cg_noalloc(NaArgs a) {
     }
     const int d = a.diag[i];
     if (ok && d != 0) ok = d >= r0 && d < r1 && a.cols[d - 1] == i + 1;
-    if (!ok) atomicExch(err, (int)EGPU_ERR_ARG);
+    if (!ok) egpu_record(err, (int)EGPU_ERR_ARG);
   }
   if (!grid_barrier(bar, err, epoch)) return;
 
