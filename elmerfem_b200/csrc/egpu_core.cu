@@ -606,6 +606,23 @@ static int pick_lpr(const egpu_mat *A) {
 
 namespace egpu {
 
+// Lets launches of a kernel use all the dynamic shared memory a block can have.  The limit is an
+// attribute of the kernel on the device, shared by all contexts and threads: set to one launch's
+// size, it would be lowered under another context's launch of the same kernel, which is then
+// refused.  Every context sets the same value, before its first such launch.
+int allow_shared(egpu_ctx *ctx, const void *kernel) {
+  auto &done = ctx->shared_allowed;
+  if (std::find(done.begin(), done.end(), kernel) != done.end()) return EGPU_OK;
+  int most = 0;
+  cudaFuncAttributes fa;
+  EGPU_CUDA_TRY(ctx, cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  EGPU_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, kernel));
+  EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          most - (int)fa.sharedSizeBytes));
+  done.push_back(kernel);
+  return EGPU_OK;
+}
+
 int ensure_ctx_scratch(egpu_ctx *ctx) {
   if (!ctx->sync.p) {
     EGPU_CUDA_TRY(ctx, ctx->sync.alloc(EGPU_SYNC_WORDS));
@@ -1755,9 +1772,7 @@ int lu_apply(egpu_mat *A, const double *v_dev, double *u_dev) {
   a.tri_per_block = tri_per_block(A, TRI_TS, ctx->num_sms * 2, EGPU_BLOCK);
   if (a.tri_cta) {
     const size_t smem = A->tri.cta_smem[0];
-    if (smem > 48 * 1024)
-      EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute((const void *)k_lu_apply_block,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024 && (rc = allow_shared(ctx, (const void *)k_lu_apply_block))) return rc;
     double *slo = A->work.p + A->ldw, *yup = A->work.p + 2 * A->ldw;
     k_gather_slots<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(n, A->tri.lower_order.p, v_dev, slo);
     k_lu_apply_block<<<1, EGPU_KBLOCK, smem, ctx->stream>>>(a, slo, yup, u_dev);
@@ -1767,8 +1782,7 @@ int lu_apply(egpu_mat *A, const double *v_dev, double *u_dev) {
     const size_t smem = range_smem_bytes<double>(a.rg_rows, a.rg_ext, a.rg_stage);
     const void *k = A->tri.rg_k == 10 ? (const void *)k_lu_apply_range<TRI_RANGE10>
                                      : (const void *)k_lu_apply_range<TRI_RANGE7>;
-    if (smem > 48 * 1024)
-      EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024 && (rc = allow_shared(ctx, k))) return rc;
     void *args[] = {&a, &v_dev, &u_dev};
     rc = cudaLaunchCooperativeKernel(k, dim3((n + a.rg_rows - 1) / a.rg_rows),
                                      dim3(EGPU_KBLOCK), args, smem, ctx->stream);

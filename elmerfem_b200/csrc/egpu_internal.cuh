@@ -132,6 +132,7 @@ struct egpu_ctx {
   unsigned int *sync_host_err = nullptr;
   // host-mapped abort word (egpu_abort): written by any host thread, polled by the kernels
   volatile int *abort_word = nullptr;
+  std::vector<const void *> shared_allowed;  // kernels this context has passed to allow_shared
 };
 
 // One triangle of the level-synchronous solve that a single block runs (CtaTri in

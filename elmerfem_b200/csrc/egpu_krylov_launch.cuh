@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "egpu_krylov.cuh"
+#include "egpu_solve.h"
 
 namespace egpu {
 
@@ -18,9 +19,10 @@ constexpr int TRI_TS = 32;
 template <typename K, typename Args>
 int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, size_t smem = 0, int most = 0) {
   int bps = 0;
-  if (smem > 48 * 1024)
-    EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
+  if (smem > 48 * 1024) {
+    const int rc = allow_shared(ctx, (const void *)kernel);
+    if (rc) return rc;
+  }
   EGPU_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, EGPU_KBLOCK, smem));
   if (bps < 1) {
     egpu_set_error(ctx, "persistent kernel does not fit on an SM");
