@@ -2523,6 +2523,24 @@ extern "C" int egpu_tri_info(egpu_mat *A, int info[6]) {
   return EGPU_OK;
 }
 
+extern "C" int egpu_tri_form(egpu_mat *A, int precision, int info[4]) {
+  if (!A || !info || (precision != EGPU_FP64 && precision != EGPU_MIXED)) return EGPU_ERR_ARG;
+  if (!A->tri_built || !A->ilu_valid) return EGPU_ERR_STATE;
+  cudaSetDevice(A->ctx->device);
+  const int v = precision == EGPU_FP64 ? 0 : 1;
+  const TriSchedule &T = A->tri;
+  info[1] = info[2] = info[3] = 0;
+  if (egpu::range_use(A, v)) {
+    info[0] = EGPU_TRI_RANGES;
+    info[1] = (A->n + T.rg_rows - 1) / T.rg_rows;
+    info[2] = T.rg_g;
+    info[3] = T.rg_k;
+  } else {
+    info[0] = egpu::cta_use(A, v) ? EGPU_TRI_ONE_BLOCK : T.bs > 1 ? EGPU_TRI_NODE_BLOCKS : EGPU_TRI_ROWS;
+  }
+  return EGPU_OK;
+}
+
 extern "C" int egpu_ilu0_download(egpu_mat *A, double *ilu_values, double *diag_scaling) {
   if (!A || !A->ilu_valid) return EGPU_ERR_STATE;
   if (A->ilu_order != 0) return EGPU_ERR_STATE;  // ILU(n > 0): egpu_ilu_download

@@ -306,6 +306,13 @@ class Matrix:
         return {"node_block": int(info[0]), "lower_levels": int(info[1]), "upper_levels": int(info[2]),
                 "max_width": int(info[3]), "single_block_fp64": bool(info[4]), "single_block_fp32": bool(info[5])}
 
+    def tri_form(self, precision: int = FP64) -> dict:
+        """The form an exact triangular solve takes in FP64 or (precision=MIXED) in the FP32 inner solves."""
+        info = np.zeros(4, np.int32)
+        check(lib().egpu_tri_form(self._h, int(precision), info.ctypes.data), self.ctx.handle, "egpu_tri_form")
+        return {"form": ("rows", "node_blocks", "one_block", "ranges")[info[0]], "ranges": int(info[1]),
+                "lanes": int(info[2]), "entries": int(info[3])}
+
     def ilut(self, tol: float, scale_system: bool = True):
         """CRS_ILUT on the (scaled) matrix: (rows, cols, diag 1-based, values with inverted U diagonal)."""
         check(lib().egpu_ilut_build(self._h, int(scale_system), float(tol)), self.ctx.handle, "egpu_ilut_build")

@@ -224,6 +224,11 @@ int egpu_lu_precondition_dev(egpu_mat *A, const double *v_dev, double *u_dev);
  * for FP64 / FP32.  EGPU_ERR_STATE before the first factorisation.  No reference
  * counterpart (the reference's CRS_LUSolve has no schedule). */
 int egpu_tri_info(egpu_mat *A, int info[6]);
+/* the form an exact triangular solve of a factorised matrix takes in a precision (EGPU_FP64, or
+ * EGPU_MIXED for the FP32 inner solves): info[0] EGPU_TRI_*; for EGPU_TRI_RANGES also info[1] ranges
+ * (one block each), info[2] lanes a row, info[3] entries a lane (0 for the other forms) */
+enum { EGPU_TRI_ROWS = 0, EGPU_TRI_NODE_BLOCKS = 1, EGPU_TRI_ONE_BLOCK = 2, EGPU_TRI_RANGES = 3 };
+int egpu_tri_form(egpu_mat *A, int precision, int info[4]);
 
 /* ---- Matrix Vector Proc hook (CRSMatrix.src:3555-3559, Load.c:734-747) ----------- */
 int egpu_mv(egpu_mat *A, const double *u, double *v);
