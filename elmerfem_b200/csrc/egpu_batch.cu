@@ -1539,8 +1539,8 @@ extern "C" int egpu_batch_create(egpu_ctx *ctx, const egpu_params *prm, egpu_bat
     delete B;
     return EGPU_ERR_ALLOC;
   }
-  cudaMemset(B->d_state.p, 0, 2 * BATCH_MAX_SYS * sizeof(SysState));
-  cudaMemset(B->d_acc.p, 0, BA_NSLOT * BATCH_MAX_SYS * sizeof(double));
+  cudaMemsetAsync(B->d_state.p, 0, 2 * BATCH_MAX_SYS * sizeof(SysState), ctx->stream);
+  cudaMemsetAsync(B->d_acc.p, 0, BA_NSLOT * BATCH_MAX_SYS * sizeof(double), ctx->stream);
   B->prm = *prm;
   B->prm.precision = EGPU_MIXED;
   if (const char *e = std::getenv("EGPU_MIXED_RESTART")) B->resume_ok = e[0] != '1';
@@ -1714,8 +1714,8 @@ static int upload_desc(egpu_batch *B) {
       d[i] = B->h_desc[i];
       r[i] = B->h_ref[i];
     }
-  EGPU_CUDA_TRY(B->ctx, cudaMemcpy(B->d_desc.p, d.data(), ns * sizeof(SysDesc), cudaMemcpyHostToDevice));
-  EGPU_CUDA_TRY(B->ctx, cudaMemcpy(B->d_ref.p, r.data(), ns * sizeof(RefDesc), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(B->ctx, egpu_copy(B->ctx, B->d_desc.p, d.data(), ns * sizeof(SysDesc), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(B->ctx, egpu_copy(B->ctx, B->d_ref.p, r.data(), ns * sizeof(RefDesc), cudaMemcpyHostToDevice));
   B->desc_dirty = false;
   return EGPU_OK;
 }
@@ -1778,7 +1778,7 @@ extern "C" int egpu_batch_step(egpu_batch *B, int *finished, int *nfinished) {
       ctx->launches++;
       B->launches++;
       // state: INIT in the parity the next chunk reads
-      EGPU_CUDA_TRY(ctx, cudaMemcpy(st.data(), B->d_state.p, 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyDeviceToHost));
+      EGPU_CUDA_TRY(ctx, egpu_copy(ctx, st.data(), B->d_state.p, 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyDeviceToHost));
       for (int i : start) {
         SysState &s = st[B->parity * BATCH_MAX_SYS + i];
         BatchSys *S = B->sys[i];
@@ -1795,7 +1795,7 @@ extern "C" int egpu_batch_step(egpu_batch *B, int *finished, int *nfinished) {
         S->phase = 2;
         S->refinements++;
       }
-      EGPU_CUDA_TRY(ctx, cudaMemcpy(B->d_state.p, st.data(), 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyHostToDevice));
+      EGPU_CUDA_TRY(ctx, egpu_copy(ctx, B->d_state.p, st.data(), 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyHostToDevice));
     }
     if (!done.empty()) {
       rc = upload_selection(B, done, &total);
@@ -1889,7 +1889,7 @@ extern "C" int egpu_batch_step(egpu_batch *B, int *finished, int *nfinished) {
     cudaEventElapsedTime(&B->last_ms, ctx->ek0, ctx->ek1);
     B->last_iters = hit[0];
     B->last_nnz = nnz_run;
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(st.data(), B->d_state.p, 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, st.data(), B->d_state.p, 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyDeviceToHost));
     std::vector<int> upd;
     for (int i = 0; i < ns; ++i) {
       BatchSys *S = B->sys[i];
@@ -1905,7 +1905,7 @@ extern "C" int egpu_batch_step(egpu_batch *B, int *finished, int *nfinished) {
       // x += ||r|| d, then the system needs a new residual
       std::vector<double> rn(ns, 0.0);
       for (int i : upd) rn[i] = B->sys[i]->rnorm;
-      EGPU_CUDA_TRY(ctx, cudaMemcpy(B->d_norms.p + BATCH_MAX_SYS, rn.data(), ns * sizeof(double), cudaMemcpyHostToDevice));
+      EGPU_CUDA_TRY(ctx, egpu_copy(ctx, B->d_norms.p + BATCH_MAX_SYS, rn.data(), ns * sizeof(double), cudaMemcpyHostToDevice));
       int total = 0;
       int rc = upload_selection(B, upd, &total);
       if (rc) return rc;
@@ -1919,7 +1919,7 @@ extern "C" int egpu_batch_step(egpu_batch *B, int *finished, int *nfinished) {
         B->sys[i]->phase = 1;
         st[B->parity * BATCH_MAX_SYS + i].status = ST_IDLE;
       }
-      EGPU_CUDA_TRY(ctx, cudaMemcpy(B->d_state.p, st.data(), 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyHostToDevice));
+      EGPU_CUDA_TRY(ctx, egpu_copy(ctx, B->d_state.p, st.data(), 2 * BATCH_MAX_SYS * sizeof(SysState), cudaMemcpyHostToDevice));
     }
   }
   if (nfinished) *nfinished = nf;

@@ -750,9 +750,9 @@ int ensure_ilu_structure(egpu_mat *A, int order) {
     A->ilu_max_row = A->max_row;
   } else {
     std::vector<int> rows(n + 1), cols(A->nnz), diag(n), r, c, d;
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(rows.data(), A->rows.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(cols.data(), A->cols.p, A->nnz * sizeof(int), cudaMemcpyDeviceToHost));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(diag.data(), A->diag.p, n * sizeof(int), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, rows.data(), A->rows.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, cols.data(), A->cols.p, A->nnz * sizeof(int), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, diag.data(), A->diag.p, n * sizeof(int), cudaMemcpyDeviceToHost));
     ::egpu_ilu_structure(n, rows, cols, diag, order, r, c, d);
     std::vector<int> scatter(A->nnz);
     int maxrow = 0;
@@ -774,10 +774,10 @@ int ensure_ilu_structure(egpu_mat *A, int order) {
     EGPU_CUDA_TRY(ctx, A->ilu_cols.alloc(A->ilu_nnz));
     EGPU_CUDA_TRY(ctx, A->ilu_diag.alloc(n));
     EGPU_CUDA_TRY(ctx, A->ilu_scatter.alloc(A->nnz));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_rows.p, r.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_cols.p, c.data(), A->ilu_nnz * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_diag.p, d.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_scatter.p, scatter.data(), A->nnz * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_rows.p, r.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_cols.p, c.data(), A->ilu_nnz * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_diag.p, d.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_scatter.p, scatter.data(), A->nnz * sizeof(int), cudaMemcpyHostToDevice));
   }
   A->ilu_order = order;
   A->tri_built = false;
@@ -857,9 +857,9 @@ int ensure_tri_schedule(egpu_mat *A) {
   // the schedules follow the ILU structure (the matrix's pattern for ILU0)
   const long long inz = A->ilu_nnz;
   std::vector<int> rows(n + 1), cols(inz), diag(n);
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(rows.data(), A->ilu_rows.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(cols.data(), A->ilu_cols.p, inz * sizeof(int), cudaMemcpyDeviceToHost));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(diag.data(), A->ilu_diag.p, n * sizeof(int), cudaMemcpyDeviceToHost));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, rows.data(), A->ilu_rows.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, cols.data(), A->ilu_cols.p, inz * sizeof(int), cudaMemcpyDeviceToHost));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, diag.data(), A->ilu_diag.p, n * sizeof(int), cudaMemcpyDeviceToHost));
   for (int i = 0; i < n; ++i)
     if (diag[i] < 0) {
       egpu_set_error(ctx, "ILU0 needs a stored diagonal in every row");
@@ -889,8 +889,8 @@ int ensure_tri_schedule(egpu_mat *A) {
   }
   EGPU_CUDA_TRY(ctx, A->tri.lower_order.alloc(n));
   EGPU_CUDA_TRY(ctx, A->tri.upper_order.alloc(n));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(A->tri.lower_order.p, lo.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(A->tri.upper_order.p, up.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->tri.lower_order.p, lo.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->tri.upper_order.p, up.data(), n * sizeof(int), cudaMemcpyHostToDevice));
   {
     // packed strictly-lower / strictly-upper parts in slot order
     std::vector<int> lp(n + 1, 0), upp(n + 1, 0), ud(n);
@@ -930,13 +930,13 @@ int ensure_tri_schedule(egpu_mat *A) {
     EGPU_CUDA_TRY(ctx, T.lo_src.alloc(ls.size()));
     EGPU_CUDA_TRY(ctx, T.up_cols.alloc(uc.size()));
     EGPU_CUDA_TRY(ctx, T.up_src.alloc(us.size()));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.lo_ptr.p, lp.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.up_ptr.p, upp.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.up_dsrc.p, ud.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.lo_cols.p, lc.data(), lc.size() * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.lo_src.p, ls.data(), ls.size() * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.up_cols.p, uc.data(), uc.size() * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(T.up_src.p, us.data(), us.size() * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.lo_ptr.p, lp.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.up_ptr.p, upp.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.up_dsrc.p, ud.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.lo_cols.p, lc.data(), lc.size() * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.lo_src.p, ls.data(), ls.size() * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.up_cols.p, uc.data(), uc.size() * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, T.up_src.p, us.data(), us.size() * sizeof(int), cudaMemcpyHostToDevice));
     // the single-block schedule needs rows sorted by row level: not with node blocks
     if (A->tri.bs == 1) {
       const int rc = build_cta_schedule(A, rows, cols, diag, lo, up, lp, lc, upp, uc);
@@ -1071,10 +1071,10 @@ int ilut_factor(egpu_mat *A, double tol) {
   EGPU_CUDA_TRY(ctx, A->ilu_cols.alloc(nz));
   EGPU_CUDA_TRY(ctx, A->ilu_diag.alloc(n));
   EGPU_CUDA_TRY(ctx, A->ilu.alloc(nz));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_rows.p, ir.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_cols.p, ic.data(), nz * sizeof(int), cudaMemcpyHostToDevice));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu_diag.p, id.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(A->ilu.p, iv.data(), nz * sizeof(double), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_rows.p, ir.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_cols.p, ic.data(), nz * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu_diag.p, id.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, A->ilu.p, iv.data(), nz * sizeof(double), cudaMemcpyHostToDevice));
   A->ilu_scatter.release();
   A->ilu_in.release();
   A->ilu_nnz = nz;
@@ -1592,7 +1592,7 @@ int solve_mixed(egpu_mat *A, const double *b_dev, double *x_dev, const egpu_para
   double bnorm_s = 1.0;
   if (!sc) {
     std::vector<double> hp(2 * nbp);
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(hp.data(), ctx->partials.p, 2 * nbp * sizeof(double), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, hp.data(), ctx->partials.p, 2 * nbp * sizeof(double), cudaMemcpyDeviceToHost));
     double t = 0.0;
     for (int i = 0; i < nbp; ++i) t += hp[nbp + i];
     bnorm_s = std::sqrt(t);
@@ -2136,15 +2136,16 @@ extern "C" int egpu_matrix_bind(egpu_ctx *ctx, int n, const int *rows, const int
         (c16 && (e = A->sell_c16.alloc(total))) || (c16 && (e = A->sell_cptr.alloc(ns))) ||
         (c16 && (e = A->sell_csc.alloc(std::max<size_t>(1, csc.size())))))
       return fail(e);
-    if (c16) {
-      cudaMemcpy(A->sell_cptr.p, cptr.data(), ns * sizeof(int), cudaMemcpyHostToDevice);
-      cudaMemcpy(A->sell_csc.p, csc.data(), csc.size() * sizeof(int16_t), cudaMemcpyHostToDevice);
-    }
-    cudaMemcpy(A->sell_ptr.p, sp.data(), ns * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(A->sell_w.p, sw.data(), ns * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(A->sell_swr.p, swr.data(), ns * sizeof(int2), cudaMemcpyHostToDevice);
-    cudaMemcpy(A->sell_cols.p, sc.data(), total * sizeof(int), cudaMemcpyHostToDevice);
-    if (c16) cudaMemcpy(A->sell_c16.p, s16.data(), total * sizeof(int16_t), cudaMemcpyHostToDevice);
+    auto put = [&](void *dst, const void *src, size_t bytes) {
+      return egpu_copy(ctx, dst, src, bytes, cudaMemcpyHostToDevice);
+    };
+    if ((c16 && (e = put(A->sell_cptr.p, cptr.data(), ns * sizeof(int)))) ||
+        (c16 && (e = put(A->sell_csc.p, csc.data(), csc.size() * sizeof(int16_t)))) ||
+        (e = put(A->sell_ptr.p, sp.data(), ns * sizeof(int))) || (e = put(A->sell_w.p, sw.data(), ns * sizeof(int))) ||
+        (e = put(A->sell_swr.p, swr.data(), ns * sizeof(int2))) ||
+        (e = put(A->sell_cols.p, sc.data(), total * sizeof(int))) ||
+        (c16 && (e = put(A->sell_c16.p, s16.data(), total * sizeof(int16_t)))))
+      return fail(e);
   }
   if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return fail(e);
   *out = A;
@@ -2496,7 +2497,7 @@ extern "C" int egpu_ilu_download(egpu_mat *A, int *ilu_rows, int *ilu_cols, int 
   std::vector<int> tmp;
   auto down1 = [&](int *dst, const int *src, long long cnt) -> int {
     tmp.resize(cnt);
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(tmp.data(), src, cnt * sizeof(int), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, tmp.data(), src, cnt * sizeof(int), cudaMemcpyDeviceToHost));
     for (long long k = 0; k < cnt; ++k) dst[k] = tmp[k] + 1;
     return EGPU_OK;
   };
@@ -2506,7 +2507,7 @@ extern "C" int egpu_ilu_download(egpu_mat *A, int *ilu_rows, int *ilu_cols, int 
   if (!rc && ilu_diag) rc = down1(ilu_diag, A->ilu_diag.p, n);
   if (rc) return rc;
   if (ilu_values)
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(ilu_values, A->ilu.p, nz * sizeof(double), cudaMemcpyDeviceToHost));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, ilu_values, A->ilu.p, nz * sizeof(double), cudaMemcpyDeviceToHost));
   return (int)nz;
 }
 

@@ -135,6 +135,16 @@ struct egpu_ctx {
   std::vector<const void *> shared_allowed;  // kernels this context has passed to allow_shared
 };
 
+// A copy between host and device memory in the order of the context's stream, complete on return.
+// cudaMemcpy and cudaMemset are in the order of the legacy stream, which the context's
+// (non-blocking) stream does not wait for and which does not wait for it; and from pageable
+// memory cudaMemcpy returns when the data is staged, before it is in place.  A kernel launched
+// next could so read what the buffer held before.
+inline cudaError_t egpu_copy(const egpu_ctx *ctx, void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, ctx->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
+}
+
 // One triangle of the level-synchronous solve that a single block runs (CtaTri in
 // egpu_krylov.cuh).  Level L owns slots [lev.x, lev.x + lev.y) and an ELL block of
 // lev.z entries per row stored column-major at [lev.w, lev.w + round8(lev.y * lev.z)):

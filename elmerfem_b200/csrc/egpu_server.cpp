@@ -115,9 +115,11 @@ int prepare(egpu_server *S, Request *r) {
   rc = egpu_matrix_update_values(r->A, r->values.data());
   if (rc) return rc;
   void *q = nullptr;
+  const cudaStream_t stream = (cudaStream_t)egpu_stream(S->ctx);  // in its order: the batch reads it there
   if (egpu::dev_alloc(&q, sizeof(double) * r->n, &r->rhs_cap, &r->rhs_devid) != cudaSuccess ||
       !(r->rhs_dev = (double *)q) ||
-      cudaMemcpy(r->rhs_dev, r->rhs.data(), sizeof(double) * r->n, cudaMemcpyHostToDevice) != cudaSuccess)
+      cudaMemcpyAsync(r->rhs_dev, r->rhs.data(), sizeof(double) * r->n, cudaMemcpyHostToDevice, stream) != cudaSuccess ||
+      cudaStreamSynchronize(stream) != cudaSuccess)
     return EGPU_ERR_ALLOC;
   return egpu_batch_add_matrix(S->batch, r->A, r->rhs_dev);
 }

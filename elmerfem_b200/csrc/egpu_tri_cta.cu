@@ -112,10 +112,10 @@ int build_cta_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vec
     EGPU_CUDA_TRY(ctx, H.ridx.alloc(T.nent));
     EGPU_CUDA_TRY(ctx, H.src.alloc(T.nent));
     EGPU_CUDA_TRY(ctx, H.map.alloc(T.map.size()));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(H.lev.p, lev.data(), lev.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(H.ridx.p, T.ridx.data(), T.nent * sizeof(uint16_t), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(H.src.p, T.src.data(), T.nent * sizeof(int), cudaMemcpyHostToDevice));
-    EGPU_CUDA_TRY(ctx, cudaMemcpy(H.map.p, T.map.data(), T.map.size() * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, H.lev.p, lev.data(), lev.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, H.ridx.p, T.ridx.data(), T.nent * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, H.src.p, T.src.data(), T.nent * sizeof(int), cudaMemcpyHostToDevice));
+    EGPU_CUDA_TRY(ctx, egpu_copy(ctx, H.map.p, T.map.data(), T.map.size() * sizeof(int), cudaMemcpyHostToDevice));
     H.nlev = T.nlev;
     H.nent = T.nent;
     return EGPU_OK;
@@ -125,8 +125,8 @@ int build_cta_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vec
   if (rc) return rc;
   EGPU_CUDA_TRY(ctx, S.pos_lo.alloc(P.pos_lo.size()));
   EGPU_CUDA_TRY(ctx, S.pos_up.alloc(P.pos_up.size()));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(S.pos_lo.p, P.pos_lo.data(), P.pos_lo.size() * sizeof(int), cudaMemcpyHostToDevice));
-  EGPU_CUDA_TRY(ctx, cudaMemcpy(S.pos_up.p, P.pos_up.data(), P.pos_up.size() * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, S.pos_lo.p, P.pos_lo.data(), P.pos_lo.size() * sizeof(int), cudaMemcpyHostToDevice));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, S.pos_up.p, P.pos_up.data(), P.pos_up.size() * sizeof(int), cudaMemcpyHostToDevice));
   S.cta_rs = P.rs;
   for (int v = 0; v < 2; ++v) {
     S.cta_ok[v] = P.fits[v];
@@ -282,7 +282,7 @@ int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::v
     auto put = [&](auto &dst, const auto &src) -> int {
       EGPU_CUDA_TRY(ctx, dst.alloc(std::max<size_t>(1, src.size())));
       if (!src.empty())
-        EGPU_CUDA_TRY(ctx, cudaMemcpy(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
+        EGPU_CUDA_TRY(ctx, egpu_copy(ctx, dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
       return EGPU_OK;
     };
     int rc = put(D.lev_ptr, T.lev_ptr);
