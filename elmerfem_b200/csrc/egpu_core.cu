@@ -476,7 +476,7 @@ static int grid_for(const egpu_ctx *ctx, long long work, int block = 256) {
 static void build_levels(int n, const std::vector<int> &rows, const std::vector<int> &cols,
                          const std::vector<int> &diag, std::vector<int> &lower,
                          std::vector<int> &upper, int &nlow, int &nup, int &maxl, int &maxu,
-                         int &maxw, std::vector<int> &lev_lo, std::vector<int> &lev_up) {
+                         int &maxw) {
   maxw = 0;
   std::vector<int> lev(n, 0);
   nlow = 0;
@@ -495,7 +495,6 @@ static void build_levels(int n, const std::vector<int> &rows, const std::vector<
   for (int l = 0; l < nlow; ++l) maxw = std::max(maxw, cnt[l + 1] - cnt[l]);
   lower.assign(n, 0);
   for (int i = 0; i < n; ++i) lower[cnt[lev[i]]++] = i;
-  lev_lo = lev;
   nup = 0;
   for (int i = n - 1; i >= 0; --i) {
     int l = 0;
@@ -510,7 +509,6 @@ static void build_levels(int n, const std::vector<int> &rows, const std::vector<
   for (int l = 0; l < nup; ++l) maxw = std::max(maxw, cnt[l + 1] - cnt[l]);
   upper.assign(n, 0);
   for (int i = n - 1; i >= 0; --i) upper[cnt[lev[i]]++] = i;
-  lev_up.swap(lev);
 }
 
 // Node blocks: the largest bs <= TRI_BS_MAX dividing n such that every aligned group of bs
@@ -547,7 +545,7 @@ static int node_block_size(int n, const std::vector<int> &rows, const std::vecto
 // by level, rows ascending inside; upper: rows descending inside).  maxw counts rows.
 static void build_block_levels(int n, int bs, const std::vector<int> &rows, const std::vector<int> &cols,
                                const std::vector<int> &diag, std::vector<int> &lower, std::vector<int> &upper,
-                               int &nlow, int &nup, int &maxw, std::vector<int> &lev_lo, std::vector<int> &lev_up) {
+                               int &nlow, int &nup, int &maxw) {
   const int nb = n / bs;
   std::vector<int> lev(nb, 0);
   nlow = nup = maxw = 0;
@@ -568,7 +566,6 @@ static void build_block_levels(int n, int bs, const std::vector<int> &rows, cons
     const int q = cnt[lev[m]]++;
     for (int k = 0; k < bs; ++k) lower[q * bs + k] = m * bs + k;
   }
-  lev_lo = lev;
   for (int m = nb - 1; m >= 0; --m) {
     int l = 0;
     for (int i = m * bs; i < (m + 1) * bs; ++i)
@@ -586,7 +583,6 @@ static void build_block_levels(int n, int bs, const std::vector<int> &rows, cons
     const int q = cnt[lev[m]]++;
     for (int k = 0; k < bs; ++k) upper[q * bs + k] = m * bs + bs - 1 - k;
   }
-  lev_up.swap(lev);
 }
 
 // lanes per row of the standalone CRS SpMV (egpu_mv)
@@ -812,17 +808,7 @@ static void view_tri(egpu_mat *A, const egpu_mat *proto) {
       T.cta_sr[v] = P.cta_sr[v];
       T.cta_smem[v] = P.cta_smem[v];
     }
-    T.rg_rows = P.rg_rows;
-    T.rg_ext = P.rg_ext;
-    T.rg_g = P.rg_g;
-    T.rg_k = P.rg_k;
-    T.rg_nt = P.rg_nt;
-    for (int v = 0; v < 2; ++v) {
-      T.rg_ok[v] = P.rg_ok[v];
-      T.rg_stage[v] = P.rg_stage[v];
-    }
-    T.rg_lo.view(P.rg_lo);
-    T.rg_up.view(P.rg_up);
+    range_view(T, P);
     T.cta_rs = P.cta_rs;
     T.pos_lo.view(P.pos_lo);
     T.pos_up.view(P.pos_up);
@@ -865,21 +851,19 @@ int ensure_tri_schedule(egpu_mat *A) {
       egpu_set_error(ctx, "ILU0 needs a stored diagonal in every row");
       return EGPU_ERR_ARG;
     }
-  std::vector<int> lo, up, lev_lo, lev_up;
+  std::vector<int> lo, up;
   build_levels(n, rows, cols, diag, lo, up, A->tri.lower_levels, A->tri.upper_levels, A->tri.max_lower,
-               A->tri.max_upper, A->tri.max_width, lev_lo, lev_up);
+               A->tri.max_upper, A->tri.max_width);
   A->tri.bs = 1;
   {
     const int bs = node_block_size(n, rows, cols, diag);
     if (bs > 1) {
-      std::vector<int> blo, bup, blev_lo, blev_up;
+      std::vector<int> blo, bup;
       int bl = 0, bu = 0, bw = 0;
-      build_block_levels(n, bs, rows, cols, diag, blo, bup, bl, bu, bw, blev_lo, blev_up);
+      build_block_levels(n, bs, rows, cols, diag, blo, bup, bl, bu, bw);
       if (tri_prefer_node_blocks(A->tri.lower_levels, A->tri.upper_levels, bl, bu, n)) {
         lo.swap(blo);
         up.swap(bup);
-        lev_lo.swap(blev_lo);
-        lev_up.swap(blev_up);
         A->tri.bs = bs;
         A->tri.lower_levels = bl;
         A->tri.upper_levels = bu;
@@ -945,8 +929,10 @@ int ensure_tri_schedule(egpu_mat *A) {
       T.cta_ok[0] = T.cta_ok[1] = false;
     }
   }
-  const int rc = build_range_schedule(A, rows, cols, diag, lev_lo, lev_up);
-  if (rc) return rc;
+  // the row ranges are planned when an exact solve asks for them (ensure_range_plan)
+  A->tri.rg_built = false;
+  A->tri.rg_rows = 0;
+  A->rg_packed[0] = A->rg_packed[1] = false;
   A->tri_built = true;
   return EGPU_OK;
 }
@@ -2529,6 +2515,8 @@ extern "C" int egpu_tri_form(egpu_mat *A, int precision, int info[4]) {
   if (!A->tri_built || !A->ilu_valid) return EGPU_ERR_STATE;
   cudaSetDevice(A->ctx->device);
   const int v = precision == EGPU_FP64 ? 0 : 1;
+  const int rc = egpu::ensure_range_plan(A, v);
+  if (rc) return rc;
   const TriSchedule &T = A->tri;
   info[1] = info[2] = info[3] = 0;
   if (egpu::range_use(A, v)) {

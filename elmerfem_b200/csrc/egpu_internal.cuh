@@ -200,10 +200,11 @@ struct TriSchedule {
   // hold whole blocks (slots s*bs .. s*bs+bs-1: lower ascending, upper descending rows) and
   // the levels count blocks
   int bs = 1;
-  // row-range schedule (egpu_tri_range.h): rows per range (0: none), external cells, lanes and
+  // row-range schedule (egpu_tri_range.h), made when an exact solve first asks for it (rg_built,
+  // whether or not the form was then chosen): rows per range (0: none), external cells, lanes and
   // entries a lane, threads solving rows, bytes of a stage; rg_ok[v]: fits in FP64 (v = 0) / FP32 (v = 1)
   int rg_rows = 0, rg_ext = 0, rg_g = 0, rg_k = 0, rg_nt = 0, rg_stage[2] = {0, 0};
-  bool rg_ok[2] = {false, false};
+  bool rg_ok[2] = {false, false}, rg_built = false;
   RangeTriDev rg_lo, rg_up;
   // level-synchronous single-block schedule; cta_ok[v] for FP64 (v = 0) / FP32 (v = 1)
   CtaTriHost cta_lo, cta_up;

@@ -61,10 +61,10 @@ int build_cta_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vec
                        const std::vector<int> &lp, const std::vector<int> &lc, const std::vector<int> &upp,
                        const std::vector<int> &uc);
 int cta_fill_values(egpu_mat *A);
-// row-range solves (egpu_tri_cta.cu): the schedule when the model prefers it, the factors packed
-// for it (v = 0 FP64, 1 FP32; once per factorisation), and whether a solve uses it
-int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vector<int> &cols,
-                         const std::vector<int> &diag, const std::vector<int> &lev_lo, const std::vector<int> &lev_up);
+// row-range solves (egpu_tri_cta.cu): the schedule, made on first need, a clone's view of it, the
+// factors packed for it (v = 0 FP64, 1 FP32; once per factorisation), and whether a solve uses it
+int ensure_range_plan(egpu_mat *A, int v);
+void range_view(TriSchedule &T, const TriSchedule &P);
 int range_alloc(egpu_mat *A, int v);
 int range_pack(egpu_mat *A, int v);
 bool range_use(const egpu_mat *A, int v);

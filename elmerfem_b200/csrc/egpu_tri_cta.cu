@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <thread>
 
 #include "egpu_krylov.cuh"
 #include "egpu_solve.h"
@@ -45,6 +46,18 @@ int tri_mode_env() {
 double est_syncfree(int nlev_lo, int nlev_up, int n) { return 0.9e-6 * (nlev_lo + nlev_up) + 0.8e-9 * 2.0 * n; }
 double est_nodeblock(int nlev_lo, int nlev_up, int n) { return 1.7e-6 * (nlev_lo + nlev_up) + 0.65e-9 * 2.0 * n; }
 double est_block(int nlev_lo, int nlev_up, int n) { return 0.6e-6 * (nlev_lo + nlev_up) + 4e-9 * 2.0 * n + 3e-6; }
+
+// rows of a range for the k-th number of ranges that is tried, largest number first; false: none
+// (EGPU_TRI_RANGES sets the only one)
+constexpr int RANGE_COUNTS = 10;
+bool range_rows_of(const egpu_ctx *ctx, int n, int bs, int k, int &per) {
+  constexpr int div[RANGE_COUNTS] = {1, 2, 3, 4, 6, 9, 12, 18, 37, 148};
+  const int forced = std::getenv("EGPU_TRI_RANGES") ? std::atoi(std::getenv("EGPU_TRI_RANGES")) : 0;
+  if (k >= RANGE_COUNTS || (forced && k > 0)) return false;
+  const int nr = std::max(1, std::min(ctx->num_sms, forced ? forced : ctx->num_sms / div[k]));
+  per = ((n + nr - 1) / nr + bs - 1) / bs * bs;
+  return true;
+}
 
 }  // namespace
 
@@ -177,12 +190,6 @@ bool cta_use(const egpu_mat *A, int v) {
   return est_block(S.cta_lo.nlev, S.cta_up.nlev, A->n) < est_syncfree(S.cta_lo.nlev, S.cta_up.nlev, A->n);
 }
 
-// Row-range solves when their modelled time (cycles at the 1.9 GHz the cards run at, plus the
-// passes over the right-hand side) beats the estimates of the other schedules.  The number of
-// ranges is the best of a few: fewer mean fewer hand-overs through L2, more mean narrower
-// levels and less shared memory.  Own values, external values and right-hand sides of a range
-// have to fit in shared memory (RANGE_SMEM of the 227 KB), in FP64 if any number of ranges
-// allows it, else in FP32 only.
 // shared-memory index of every padded entry (by global slot): the own row's slot, an external
 // row's cell, or the zero cell
 template <bool LOWER>
@@ -219,16 +226,35 @@ __global__ void k_range_index(int n, int bs, int per, int gk, int zero, const in
 constexpr size_t RANGE_SMEM = 216 * 1024;
 constexpr double RANGE_PASSES = 8e-6;
 
-int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vector<int> &cols,
-                         const std::vector<int> &diag, const std::vector<int> &lev_lo,
-                         const std::vector<int> &lev_up) {
+namespace {
+
+// one number of ranges: its plan and modelled time; fit 0: shared memory holds it in FP64, 1: in
+// FP32 only, 2: neither
+struct RangeChoice {
+  int per = 0, fit = 2;
+  double t = 0.0;
+  plan::RangeTriHost lo, up;
+};
+
+}  // namespace
+
+// Row-range solves when their modelled time (cycles at the 1.9 GHz the cards run at, plus the
+// passes over the right-hand side) beats the estimates of the other schedules.  The number of
+// ranges is the best of a few: fewer mean fewer hand-overs through L2, more mean narrower
+// levels and less shared memory.  Own values, external values and right-hand sides of a range
+// have to fit in shared memory (RANGE_SMEM of the 227 KB), in FP64 if any number of ranges
+// allows it, else in FP32 only.
+//
+// The plan is host work (hex 64^3: 14 ms of counting and 9 ms of modelling a triangle and number of
+// ranges), so the numbers are tried side by side, each on a thread, and one whose model without
+// external values is too slow already is dropped before it is planned.  First exact solve less
+// second, 16-core host: hex 32^3 12 ms, 64^3 93 ms, 96^3 240 ms, elasticity 64^3 (form not taken)
+// 243 ms; one after another 100, 470, 900 and 900 ms and more.
+static int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::vector<int> &cols,
+                                const std::vector<int> &diag) {
   egpu_ctx *ctx = A->ctx;
   TriSchedule &S = A->tri;
   const int n = A->n, bs = S.bs, mode = tri_mode_env();
-  S.rg_rows = 0;
-  S.rg_ok[0] = S.rg_ok[1] = false;
-  A->rg_packed[0] = A->rg_packed[1] = false;
-  if (mode == 1 || mode == 2) return EGPU_OK;
   int most = 0;
   for (int r = 0; r < n; r += bs) {
     int beg, ne;
@@ -239,42 +265,66 @@ int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::v
   }
   const plan::RangeShape sh = plan::range_shape(most);
   if (sh.g == 0) return EGPU_OK;
-  const int forced = std::getenv("EGPU_TRI_RANGES") ? std::atoi(std::getenv("EGPU_TRI_RANGES")) : 0;
-  plan::RangeTriHost lo, up, best_lo, best_up;
-  double best = 0.0;
-  int best_per = 0, best_fit = 2;
-  for (int div : {1, 2, 3, 4, 6, 9, 12, 18, 37, 148}) {
-    if (forced && div > 1) break;
-    const int nr = std::max(1, std::min(ctx->num_sms, forced ? forced : ctx->num_sms / div));
-    const int per = ((n + nr - 1) / nr + bs - 1) / bs * bs;
-    if (range_smem_bytes<float>(per, 0, 0) > RANGE_SMEM || per > 32000) break;
-    if (!plan::range_triangle(n, bs, per, sh, true, rows, cols, diag, lev_lo, lo) ||
-        !plan::range_triangle(n, bs, per, sh, false, rows, cols, diag, lev_up, up))
-      continue;
-    const int ext = std::max(lo.max_ext, up.max_ext), maxr = std::max(lo.max_rows, up.max_rows);
-    auto bytes = [&](int vsize) { return plan::range_record(maxr, sh.g * sh.k, vsize); };
-    const int fit = range_smem_bytes<double>(per, ext, bytes(8)) <= RANGE_SMEM  ? 0
-                    : range_smem_bytes<float>(per, ext, bytes(4)) <= RANGE_SMEM ? 1
-                                                                                : 2;
-    if (fit == 2 || fit > best_fit) continue;
-    const double t = (plan::range_cycles(n, bs, per, sh, ext, true, rows, cols, diag, lev_lo) +
-                      plan::range_cycles(n, bs, per, sh, ext, false, rows, cols, diag, lev_up)) / 1.9e9 + RANGE_PASSES;
-    if (best_per == 0 || fit < best_fit || t < best) {
-      best = t;
-      best_per = per;
-      best_fit = fit;
-      std::swap(lo, best_lo);
-      std::swap(up, best_up);
-    }
-  }
-  if (best_per == 0) return EGPU_OK;
+  std::vector<int> lev_lo, lev_up;
+  plan::range_levels(n, bs, true, rows, cols, lev_lo);
+  plan::range_levels(n, bs, false, rows, cols, lev_up);
   // measured per application: sync-free 0.8 us a level + 0.24 ns a row, node blocks 1.25 us +
   // 0.4 ns (hex 32^3 372 us, 96^3 1,335 us; elasticity 24^3 440 us, 64^3 1,430 us), where the
   // row ranges take 185, 1,090, 230 and 1,600 us
   const double levels = S.lower_levels + S.upper_levels;
-  double other = bs > 1 ? 1.25e-6 * levels + 0.4e-9 * n : 0.8e-6 * levels + 0.24e-9 * n;
+  const double spread = bs > 1 ? 1.25e-6 * levels + 0.4e-9 * n : 0.8e-6 * levels + 0.24e-9 * n;
+  constexpr double SCATTER = 1.15;  // the model's
+  auto seconds = [&](int per, int ext) {
+    return (plan::range_cycles(n, bs, per, sh, ext, true, rows, cols, diag, lev_lo) +
+            plan::range_cycles(n, bs, per, sh, ext, false, rows, cols, diag, lev_up)) / 1.9e9 + RANGE_PASSES;
+  };
+  auto evaluate = [&](RangeChoice &c) {
+    if (mode != 3 && SCATTER * seconds(c.per, 0) >= spread) return;
+    if (!plan::range_triangle(n, bs, c.per, sh, true, rows, cols, diag, lev_lo, c.lo) ||
+        !plan::range_triangle(n, bs, c.per, sh, false, rows, cols, diag, lev_up, c.up))
+      return;
+    const int ext = std::max(c.lo.max_ext, c.up.max_ext), maxr = std::max(c.lo.max_rows, c.up.max_rows);
+    auto bytes = [&](int vsize) { return plan::range_record(maxr, sh.g * sh.k, vsize); };
+    if (range_smem_bytes<float>(c.per, ext, bytes(4)) > RANGE_SMEM) return;
+    c.t = seconds(c.per, ext);
+    c.fit = range_smem_bytes<double>(c.per, ext, bytes(8)) <= RANGE_SMEM ? 0 : 1;
+  };
+  std::vector<RangeChoice> choices(RANGE_COUNTS);
+  size_t nc = 0;
+  for (; nc < choices.size() && range_rows_of(ctx, n, bs, (int)nc, choices[nc].per); ++nc)
+    if (range_smem_bytes<float>(choices[nc].per, 0, 0) > RANGE_SMEM || choices[nc].per > 32000) break;
+  choices.resize(nc);
+  {
+    std::vector<std::thread> threads;
+    for (RangeChoice &c : choices) {
+      auto run = [&evaluate, &c] {
+        try {
+          evaluate(c);
+        } catch (...) {  // out of host memory: not chosen
+          c.fit = 2;
+        }
+      };
+      if (&c == &choices.back()) {
+        run();
+        break;
+      }
+      try {
+        threads.emplace_back(run);
+      } catch (...) {  // no more threads: here
+        run();
+      }
+    }
+    for (std::thread &t : threads) t.join();
+  }
+  const RangeChoice *best = nullptr;
+  for (const RangeChoice &c : choices)
+    if (c.fit < 2 && (!best || c.fit < best->fit || (c.fit == best->fit && c.t < best->t))) best = &c;
+  if (!best) return EGPU_OK;
+  const plan::RangeTriHost &best_lo = best->lo, &best_up = best->up;
+  const int best_per = best->per, best_fit = best->fit;
+  double other = spread;
   if (S.cta_ok[best_fit]) other = std::min(other, est_block(S.cta_lo.nlev, S.cta_up.nlev, n));
-  if (mode != 3 && 1.15 * best >= other) return EGPU_OK;  // the model's scatter
+  if (mode != 3 && SCATTER * best->t >= other) return EGPU_OK;
   const int ext = std::max(best_lo.max_ext, best_up.max_ext);
   const int gk = sh.g * sh.k;
   auto upload = [&](const plan::RangeTriHost &T, bool lower, RangeTriDev &D) -> int {
@@ -341,6 +391,51 @@ int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const std::v
   return EGPU_OK;
 }
 
+void range_view(TriSchedule &T, const TriSchedule &P) {
+  T.rg_rows = P.rg_rows;
+  T.rg_ext = P.rg_ext;
+  T.rg_g = P.rg_g;
+  T.rg_k = P.rg_k;
+  T.rg_nt = P.rg_nt;
+  for (int v = 0; v < 2; ++v) {
+    T.rg_ok[v] = P.rg_ok[v];
+    T.rg_stage[v] = P.rg_stage[v];
+  }
+  T.rg_built = P.rg_built;
+  T.rg_lo.view(P.rg_lo);
+  T.rg_up.view(P.rg_up);
+}
+
+// Makes the row-range plan of the ILU structure if it is not made yet; called before an exact
+// triangular solve in precision v and by nothing else, so that batches, Jacobi sweeps and
+// matrices that are only factorised do not pay for it.  An ILUT factor has a new structure
+// with every factorisation and is planned only where the form is asked for (EGPU_TRI_MODE=range):
+// the plan costs more than one solve gains.
+int ensure_range_plan(egpu_mat *A, int v) {
+  TriSchedule &S = A->tri;
+  const int mode = tri_mode_env();
+  if (!A->tri_built || S.rg_built || mode == 1 || mode == 2) return EGPU_OK;
+  if (A->ilu_order == ILU_ORDER_T && mode != 3) return EGPU_OK;
+  egpu_ctx *ctx = A->ctx;
+  const int n = A->n;
+  int per = 0;  // of the most ranges: what FP64 cannot hold there, it can hold nowhere
+  if (v == 0 && range_rows_of(ctx, n, S.bs, 0, per) && range_smem_bytes<double>(per, 0, 0) > RANGE_SMEM) return EGPU_OK;
+  if (A->parent) {  // a clone shares its prototype's plan
+    const int rc = ensure_range_plan(A->parent, v);
+    if (rc) return rc;
+    range_view(S, A->parent->tri);
+    return EGPU_OK;
+  }
+  std::vector<int> rows(n + 1), cols(A->ilu_nnz), diag(n);
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, rows.data(), A->ilu_rows.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, cols.data(), A->ilu_cols.p, A->ilu_nnz * sizeof(int), cudaMemcpyDeviceToHost));
+  EGPU_CUDA_TRY(ctx, egpu_copy(ctx, diag.data(), A->ilu_diag.p, n * sizeof(int), cudaMemcpyDeviceToHost));
+  const int rc = build_range_schedule(A, rows, cols, diag);
+  if (rc) return rc;
+  S.rg_built = true;
+  return EGPU_OK;
+}
+
 bool range_use(const egpu_mat *A, int v) {
   const int mode = tri_mode_env();
   return A->tri.rg_rows > 0 && A->tri.rg_ok[v] && mode != 1 && mode != 2;
@@ -398,7 +493,9 @@ __global__ void k_range_pack(int n, int bs, int per, int g, int gk, const int *_
 
 // the record buffers of a precision, and its packing kernels loaded
 int range_alloc(egpu_mat *A, int v) {
-  if (!A->tri_built || !range_use(A, v)) return EGPU_OK;
+  if (!A->tri_built) return EGPU_OK;
+  const int rc = ensure_range_plan(A, v);
+  if (rc || !range_use(A, v)) return rc;
   egpu_ctx *ctx = A->ctx;
   EGPU_CUDA_TRY(ctx, A->rg_lo_rec[v].alloc(A->tri.rg_lo.bytes[v]));
   EGPU_CUDA_TRY(ctx, A->rg_up_rec[v].alloc(A->tri.rg_up.bytes[v]));
@@ -431,7 +528,8 @@ static int range_pack_as(egpu_mat *A, int v) {
 }
 
 int range_pack(egpu_mat *A, int v) {
-  if (!range_use(A, v) || A->rg_packed[v]) return EGPU_OK;
+  const int rc = ensure_range_plan(A, v);
+  if (rc || !range_use(A, v) || A->rg_packed[v]) return rc;
   return v == 0 ? range_pack_as<double>(A, v) : range_pack_as<float>(A, v);
 }
 

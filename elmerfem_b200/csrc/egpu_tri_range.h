@@ -85,6 +85,25 @@ inline void range_entries(int bs, bool lower, const std::vector<int> &rows, cons
   ne = lower ? e_lo : len - e_lo - bs;
 }
 
+// dependency levels of the rows (bs == 1) or node blocks; returns their number
+inline int range_levels(int n, int bs, bool lower, const std::vector<int> &rows, const std::vector<int> &cols,
+                        std::vector<int> &lev) {
+  const int nb = n / bs;
+  int nl = 0;
+  lev.assign(nb, 0);
+  for (int q = 0; q < nb; ++q) {
+    const int m = lower ? q : nb - 1 - q;
+    int l = 0;
+    for (int e = rows[m * bs]; e < rows[m * bs + 1]; ++e) {
+      const int d = cols[e] / bs;
+      if (lower ? d < m : d > m) l = std::max(l, lev[d] + 1);
+    }
+    lev[m] = l;
+    nl = std::max(nl, l + 1);
+  }
+  return nl;
+}
+
 // Cycles of the plan's timing model, fitted to B200 measurements (hex 16^3 to 96^3, 3-DOF hex 24^3
 // to 64^3, a randomly numbered tet mesh): a level costs the FP64 units' latency through its sums
 // plus its record's way through shared memory; a value handed from one block to another a store,
