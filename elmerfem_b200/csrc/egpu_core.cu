@@ -2243,9 +2243,13 @@ extern "C" int egpu_matrix_prepare(egpu_mat *A, const egpu_params *prm) {
   if (!A || !prm || prm->precond < EGPU_PREC_NONE || prm->precond > EGPU_PREC_ILUT) return EGPU_ERR_ARG;
   cudaSetDevice(A->ctx->device);
   if (prm->precond != EGPU_PREC_ILU0) return EGPU_OK;  // ILUT: its structure needs the values
-  const int rc = egpu::ensure_ilu_structure(A, prm->ilu_order);
+  int rc = egpu::ensure_ilu_structure(A, prm->ilu_order);
+  if (!rc) rc = egpu::ensure_tri_schedule(A);
   if (rc) return rc;
-  return egpu::ensure_tri_schedule(A);
+  // the row ranges, unless the solves will be by Jacobi sweeps
+  const bool fp64 = prm->precision != EGPU_MIXED || (prm->method != EGPU_CG && prm->method != EGPU_BICGSTAB);
+  if (!fp64 && prm->method == EGPU_BICGSTAB && prm->ilu_order == 0 && prm->ilu_sweeps > 0) return EGPU_OK;
+  return egpu::ensure_range_plan(A, fp64 ? 0 : 1);
 }
 
 // device bytes a solve of this matrix holds (values, scaled and FP32 copies, factors,

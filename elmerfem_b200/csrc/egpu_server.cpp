@@ -361,7 +361,12 @@ extern "C" int egpu_server_pattern(egpu_server *S, int n, const int *rows, const
   {
     std::lock_guard<std::mutex> g(S->gpu_mu);
     int rc = egpu_matrix_bind(S->ctx, n, rows, cols, diag, zero.data(), &P.proto);
-    if (!rc) rc = egpu_matrix_prepare(P.proto, &S->prm);
+    // a batch solves by Jacobi sweeps or by triangular solves of its own: no row ranges for it
+    egpu_params batched = S->prm;
+    batched.precision = EGPU_MIXED;
+    batched.method = EGPU_BICGSTAB;
+    batched.ilu_sweeps = 1;
+    if (!rc) rc = egpu_matrix_prepare(P.proto, &batched);
     if (rc) {
       if (P.proto) egpu_matrix_free(P.proto);
       return rc;

@@ -407,8 +407,8 @@ void range_view(TriSchedule &T, const TriSchedule &P) {
 }
 
 // Makes the row-range plan of the ILU structure if it is not made yet; called before an exact
-// triangular solve in precision v and by nothing else, so that batches, Jacobi sweeps and
-// matrices that are only factorised do not pay for it.  An ILUT factor has a new structure
+// triangular solve in precision v, or where one is prepared, and by nothing else, so that
+// batches, Jacobi sweeps and matrices that are only factorised do not pay for it.  An ILUT factor has a new structure
 // with every factorisation and is planned only where the form is asked for (EGPU_TRI_MODE=range):
 // the plan costs more than one solve gains.
 int ensure_range_plan(egpu_mat *A, int v) {

@@ -21,7 +21,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import meshgen
-from .solver import PREC_ILU0, Batch, Context, Matrix, SolverParams, create_matrix
+from .solver import BICGSTAB, MIXED, PREC_ILU0, Batch, Context, Matrix, SolverParams, create_matrix
 
 
 @dataclass
@@ -85,7 +85,7 @@ class MeshPrototype:
     preconditioner given, its one-time structures are built here too.  built: (mesh, pattern)
     from build_meshes, else both are made here."""
 
-    def __init__(self, ctx: Context, m: int, precond: int | None = None, built: tuple | None = None):
+    def __init__(self, ctx: Context, m: int, precond: "SolverParams | int | None" = None, built: tuple | None = None):
         self.m = m
         if built is None:
             built = (meshgen.hex_cube(m), None)
@@ -112,7 +112,9 @@ class SolveServer:
 
     def prototype(self, m: int) -> MeshPrototype:
         if m not in self.protos:
-            self.protos[m] = MeshPrototype(self.ctx, m, self.params.precond)
+            # a batch solves by Jacobi sweeps or by triangular solves of its own: no row ranges for it
+            self.protos[m] = MeshPrototype(self.ctx, m, SolverParams(method=BICGSTAB, precond=self.params.precond,
+                                                                     precision=MIXED, ilu_sweeps=1))
         return self.protos[m]
 
     def footprint(self, req: Request) -> float:

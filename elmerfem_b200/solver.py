@@ -279,8 +279,8 @@ class Matrix:
 
     # ---- preconditioner state (A%ILUValues, A%DiagScaling)
     def prepare(self, params: "SolverParams | int"):
-        """One-time preconditioner structures (ILU(n) fill and level schedules) before the first
-        solve; params is a SolverParams or a preconditioner code (ILU order 0)."""
+        """One-time preconditioner structures (ILU(n) fill, level schedules, row ranges of exact solves)
+        before the first solve; params is a SolverParams or a preconditioner code (ILU order 0)."""
         if not isinstance(params, SolverParams):
             params = SolverParams(precond=int(params))
         prm = params.to_c()

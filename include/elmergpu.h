@@ -177,8 +177,8 @@ void egpu_matrix_free(egpu_mat *A);
  * clones; the shared data goes with the last of them. */
 int egpu_matrix_clone(egpu_mat *proto, egpu_mat **out);
 /* Builds the preconditioner's one-time structures before the first solve (for ILU(n) the
- * fill structure and the level schedules of the triangular solves; nothing for Diagonal /
- * None), so that the first IterSolver call on a pattern costs what later ones do.  Clones
+ * fill structure, the level schedules of the triangular solves and, unless prm asks for Jacobi
+ * sweeps, their row ranges; nothing for Diagonal / None), so that the first IterSolver call on a pattern costs what later ones do.  Clones
  * share their prototype's. */
 int egpu_matrix_prepare(egpu_mat *A, const egpu_params *prm);
 /* device bytes a solve of A holds beyond the shared pattern, for the given preconditioner */

@@ -1,5 +1,5 @@
-"""When the row ranges of the triangular solves are planned: by the first exact solve of a precision that
-they can serve, and by nothing else.  The plan's two index kernels show in the launch count."""
+"""When the row ranges of the triangular solves are planned: by the preparation or the first exact solve
+of a precision that they can serve, and by nothing else.  The plan's two index kernels show in the launch count."""
 import pytest
 
 import elmerfem_b200 as eg
@@ -26,10 +26,25 @@ def _default_forms(monkeypatch):
     monkeypatch.setenv("EGPU_MIXED_AUTO", "0")
 
 
-def test_preparation_and_factorisation_plan_nothing(ctx):
+def test_preparation_for_exact_solves_plans(ctx):
+    """After it, the first solve on a pattern costs what later ones do."""
+    for prm in (dict(), dict(precision=eg.MIXED, ilu_sweeps=0), dict(precision=eg.MIXED)):
+        p, v, b, A = _matrix(ctx)
+        n0 = _launches(ctx)
+        A.prepare(eg.SolverParams(method=eg.BICGSTAB, precond=eg.PREC_ILU0, **prm))
+        assert _launches(ctx) - n0 == 2
+        A.ilu0()
+        n0 = _launches(ctx)
+        assert A.tri_form(prm.get("precision", eg.FP64))["form"] == "ranges"
+        assert _launches(ctx) == n0
+        A.free()
+
+
+def test_factorisation_plans_nothing(ctx):
     p, v, b, A = _matrix(ctx)
-    A.prepare(eg.SolverParams(method=eg.BICGSTAB, precond=eg.PREC_ILU0))
     n0 = _launches(ctx)
+    A.prepare(eg.SolverParams(method=eg.BICGSTAB, precond=eg.PREC_ILU0, precision=eg.MIXED, ilu_sweeps=2))
+    assert _launches(ctx) == n0
     ilu, _ = A.ilu0()
     n1 = _launches(ctx)
     assert A.tri_form()["form"] == "ranges"
