@@ -2253,7 +2253,8 @@ extern "C" int egpu_matrix_prepare(egpu_mat *A, const egpu_params *prm) {
 }
 
 // device bytes a solve of this matrix holds (values, scaled and FP32 copies, factors,
-// work vectors), excluding the shared pattern: the admission footprint
+// work vectors), excluding the shared pattern: the admission footprint.  Batches and the server
+// never plan row ranges, so their prototypes count none.
 extern "C" long long egpu_matrix_footprint(const egpu_mat *A, int precond) {
   if (!A) return EGPU_ERR_ARG;
   const long long z = A->nnz, zs = A->sell_nnz, n = A->n, l = A->ldw;
@@ -2266,6 +2267,8 @@ extern "C" long long egpu_matrix_footprint(const egpu_mat *A, int precond) {
     b += 12 * zi + 12 * n;                                 // factors packed in solve order, FP64 + FP32
     b += 4 * zs + 4 * n;                                   // FP32 factors in SELL order (Jacobi sweeps)
     b += 12 * (A->tri.cta_lo.nent + A->tri.cta_up.nent);   // single-block layout
+    for (int v = 0; v < 2; ++v)                            // level records of the row ranges, once planned
+      if (A->tri.rg_rows > 0 && A->tri.rg_ok[v]) b += A->tri.rg_lo.bytes[v] + A->tri.rg_up.bytes[v];
   }
   return b + 8 * n;                         // back-scaled solution
 }

@@ -97,3 +97,20 @@ def test_clones_share_one_plan(ctx):
         assert rel(M.lu_precondition(b), ref) < 1e-13
     for M in (B, C, A):
         M.free()
+
+
+def test_footprint_counts_the_level_records(ctx):
+    """A solve in row ranges holds the level records of its precision: per row and padded entry an index of
+    two bytes and a value of eight or four, in both triangles."""
+    p, v, b, A = _matrix(ctx)
+    A.ilu0()
+    none = A.footprint(eg.PREC_NONE)
+    before = A.footprint(eg.PREC_ILU0)
+    form = A.tri_form()
+    assert form["form"] == "ranges"
+    extra = A.footprint(eg.PREC_ILU0) - before
+    entries = 2 * p.n * form["lanes"] * form["entries"]
+    least = entries * (10 + 6)
+    assert least <= extra <= 1.3 * least  # row numbers, headers and padding besides
+    assert A.footprint(eg.PREC_NONE) == none
+    A.free()
