@@ -932,7 +932,7 @@ int ensure_tri_schedule(egpu_mat *A) {
   // the row ranges are planned when an exact solve asks for them (ensure_range_plan)
   A->tri.rg_built = false;
   A->tri.rg_rows = 0;
-  A->rg_packed[0] = A->rg_packed[1] = false;
+  A->rg_packed[0] = A->rg_packed[1] = A->rg_off[0] = A->rg_off[1] = false;
   A->tri_built = true;
   return EGPU_OK;
 }

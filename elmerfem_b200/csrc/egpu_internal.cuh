@@ -170,6 +170,17 @@ struct RangeTriDev {
   DevBuf<long long> offset[2];
   long long bytes[2] = {0, 0};
   DevBuf<uint16_t> slot, idx;
+  void release() {
+    lev_ptr.release();
+    row.release();
+    slot_lev.release();
+    ext_ptr.release();
+    ext.release();
+    lev.release();
+    for (int v = 0; v < 2; ++v) offset[v].release();
+    slot.release();
+    idx.release();
+  }
   void view(const RangeTriDev &o) {
     lev_ptr.view(o.lev_ptr);
     row.view(o.row);
@@ -257,6 +268,7 @@ struct egpu_mat {
   // the level records of the row-range solves, packed when a solve first needs them (rg_packed[v])
   DevBuf<unsigned char> rg_lo_rec[2], rg_up_rec[2];
   bool rg_packed[2] = {false, false};
+  bool rg_off[2] = {false, false};  // no memory for the records: the other forms solve
   DevBuf<int16_t> cols16;        // column offsets (col - row) when |col-row| < 32768
   DevBuf<int> ilu_done;          // factorisation completion flags
   // SELL-32 copy of the pattern (slice s = rows 32s..32s+31, entry (k, lane) at

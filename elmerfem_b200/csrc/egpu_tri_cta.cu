@@ -228,6 +228,19 @@ constexpr double RANGE_PASSES = 8e-6;
 
 namespace {
 
+// The form is a choice: where its buffers do not fit the free device memory, the solve takes
+// another form, whose buffers it has anyway.  EGPU_ERR_ALLOC for that, else EGPU_ERR_CUDA
+template <typename T>
+int range_buffer(egpu_ctx *ctx, DevBuf<T> &b, size_t count) {
+  const cudaError_t e = b.alloc(count);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // not sticky
+    return EGPU_ERR_ALLOC;
+  }
+  EGPU_CUDA_TRY(ctx, e);
+  return EGPU_OK;
+}
+
 // one number of ranges: its plan and modelled time; fit 0: shared memory holds it in FP64, 1: in
 // FP32 only, 2: neither
 struct RangeChoice {
@@ -330,9 +343,9 @@ static int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const
   auto upload = [&](const plan::RangeTriHost &T, bool lower, RangeTriDev &D) -> int {
     static_assert(sizeof(plan::RangeLevel) == sizeof(int2), "levels are read as int2");
     auto put = [&](auto &dst, const auto &src) -> int {
-      EGPU_CUDA_TRY(ctx, dst.alloc(std::max<size_t>(1, src.size())));
-      if (!src.empty())
-        EGPU_CUDA_TRY(ctx, egpu_copy(ctx, dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
+      const int rc = range_buffer(ctx, dst, std::max<size_t>(1, src.size()));
+      if (rc || src.empty()) return rc;
+      EGPU_CUDA_TRY(ctx, egpu_copy(ctx, dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
       return EGPU_OK;
     };
     int rc = put(D.lev_ptr, T.lev_ptr);
@@ -359,8 +372,8 @@ static int build_range_schedule(egpu_mat *A, const std::vector<int> &rows, const
     }
     DevBuf<int2> ds;
     rc = put(ds, sorted);
+    if (!rc) rc = range_buffer(ctx, D.idx, (size_t)n * gk);
     if (rc) return rc;
-    EGPU_CUDA_TRY(ctx, D.idx.alloc((size_t)n * gk));
     const int grid = (int)std::max(1LL, std::min(((long long)n * gk + 255) / 256, (long long)ctx->num_sms * 32));
     if (lower)
       k_range_index<true><<<grid, 256, 0, ctx->stream>>>(n, bs, best_per, gk, best_per + ext, D.row.p, D.slot.p,
@@ -431,14 +444,19 @@ int ensure_range_plan(egpu_mat *A, int v) {
   EGPU_CUDA_TRY(ctx, egpu_copy(ctx, cols.data(), A->ilu_cols.p, A->ilu_nnz * sizeof(int), cudaMemcpyDeviceToHost));
   EGPU_CUDA_TRY(ctx, egpu_copy(ctx, diag.data(), A->ilu_diag.p, n * sizeof(int), cudaMemcpyDeviceToHost));
   const int rc = build_range_schedule(A, rows, cols, diag);
-  if (rc) return rc;
+  if (rc == EGPU_ERR_ALLOC) {
+    S.rg_lo.release();
+    S.rg_up.release();
+  } else if (rc) {
+    return rc;
+  }
   S.rg_built = true;
   return EGPU_OK;
 }
 
 bool range_use(const egpu_mat *A, int v) {
   const int mode = tri_mode_env();
-  return A->tri.rg_rows > 0 && A->tri.rg_ok[v] && mode != 1 && mode != 2;
+  return A->tri.rg_rows > 0 && A->tri.rg_ok[v] && !A->rg_off[v] && mode != 1 && mode != 2;
 }
 
 // The level records of a triangle (plan::RangeLevel) with the factors' values.  bs > 1: row k of a
@@ -494,11 +512,18 @@ __global__ void k_range_pack(int n, int bs, int per, int g, int gk, const int *_
 // the record buffers of a precision, and its packing kernels loaded
 int range_alloc(egpu_mat *A, int v) {
   if (!A->tri_built) return EGPU_OK;
-  const int rc = ensure_range_plan(A, v);
+  int rc = ensure_range_plan(A, v);
   if (rc || !range_use(A, v)) return rc;
   egpu_ctx *ctx = A->ctx;
-  EGPU_CUDA_TRY(ctx, A->rg_lo_rec[v].alloc(A->tri.rg_lo.bytes[v]));
-  EGPU_CUDA_TRY(ctx, A->rg_up_rec[v].alloc(A->tri.rg_up.bytes[v]));
+  rc = range_buffer(ctx, A->rg_lo_rec[v], A->tri.rg_lo.bytes[v]);
+  if (!rc) rc = range_buffer(ctx, A->rg_up_rec[v], A->tri.rg_up.bytes[v]);
+  if (rc == EGPU_ERR_ALLOC) {
+    A->rg_lo_rec[v].release();
+    A->rg_up_rec[v].release();
+    A->rg_off[v] = true;
+    return EGPU_OK;
+  }
+  if (rc) return rc;
   cudaFuncAttributes fa;
   EGPU_CUDA_TRY(ctx, v == 0 ? cudaFuncGetAttributes(&fa, k_range_pack<double, true>)
                             : cudaFuncGetAttributes(&fa, k_range_pack<float, true>));
@@ -514,7 +539,7 @@ static int range_pack_as(egpu_mat *A, int v) {
   const int gk = S.rg_g * S.rg_k;
   const int grid = (int)std::max(1LL, std::min(((long long)A->n * gk + 255) / 256, (long long)ctx->num_sms * 32));
   const int rc = range_alloc(A, v);
-  if (rc) return rc;
+  if (rc || !range_use(A, v)) return rc;
   k_range_pack<VT, true><<<grid, 256, 0, ctx->stream>>>(
       A->n, S.bs, S.rg_rows, S.rg_g, gk, S.rg_lo.row.p, S.rg_lo.slot_lev.p, S.rg_lo.lev.p, S.rg_lo.offset[v].p,
       S.rg_lo.idx.p, A->ilu_rows.p, A->ilu_diag.p, A->ilu.p, A->rg_lo_rec[v].p);
