@@ -602,20 +602,50 @@ static int pick_lpr(const egpu_mat *A) {
 
 namespace egpu {
 
+static egpu_ctx::KernelUse &kernel_use(egpu_ctx *ctx, const void *kernel) {
+  for (auto &u : ctx->kernel_uses)
+    if (u.kernel == kernel) return u;
+  ctx->kernel_uses.push_back({kernel, false, 0, 0});
+  return ctx->kernel_uses.back();
+}
+
 // Lets launches of a kernel use all the dynamic shared memory a block can have.  The limit is an
 // attribute of the kernel on the device, shared by all contexts and threads: set to one launch's
 // size, it would be lowered under another context's launch of the same kernel, which is then
 // refused.  Every context sets the same value, before its first such launch.
 int allow_shared(egpu_ctx *ctx, const void *kernel) {
-  auto &done = ctx->shared_allowed;
-  if (std::find(done.begin(), done.end(), kernel) != done.end()) return EGPU_OK;
+  auto &use = kernel_use(ctx, kernel);
+  if (use.shared_allowed) return EGPU_OK;
   int most = 0;
   cudaFuncAttributes fa;
   EGPU_CUDA_TRY(ctx, cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   EGPU_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, kernel));
   EGPU_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           most - (int)fa.sharedSizeBytes));
-  done.push_back(kernel);
+  use.shared_allowed = true;
+  return EGPU_OK;
+}
+
+// Blocks of a persistent Krylov kernel that an SM holds.  Asked once per context, kernel and size of
+// shared memory (a solve launches its kernel once per refinement); the first question loads the
+// kernel.
+int kernel_blocks(egpu_ctx *ctx, const void *kernel, size_t smem, int *bps) {
+  auto &use = kernel_use(ctx, kernel);
+  if (use.bps == 0 || use.smem != smem) {
+    if (smem > 48 * 1024) {
+      const int rc = allow_shared(ctx, kernel);
+      if (rc) return rc;
+    }
+    int b = 0;
+    EGPU_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, EGPU_KBLOCK, smem));
+    if (b < 1) {
+      egpu_set_error(ctx, "persistent kernel does not fit on an SM");
+      return EGPU_ERR_CUDA;
+    }
+    use.smem = smem;
+    use.bps = b;
+  }
+  *bps = use.bps;
   return EGPU_OK;
 }
 
@@ -1164,8 +1194,9 @@ static int tri_per_block(const egpu_mat *A, int lpr, int grid, int block = EGPU_
   return std::max(1, std::min(per_block_max, (want + grid - 1) / grid));
 }
 
+// launches the Krylov kernel that the solve takes, or (load) only loads it
 template <typename VT>
-static int run_krylov(egpu_mat *A, const KArgs<VT> &a0, int method, bool offs) {
+static int run_krylov(egpu_mat *A, const KArgs<VT> &a0, int method, bool offs, bool load = false) {
   egpu_ctx *ctx = A->ctx;
   KArgs<VT> a = a0;
   a.tri_per_block = tri_per_block(A, TRI_TS, ctx->num_sms);
@@ -1173,11 +1204,11 @@ static int run_krylov(egpu_mat *A, const KArgs<VT> &a0, int method, bool offs) {
   const size_t smem = a.tri_cta ? A->tri.cta_smem[sizeof(VT) == 8 ? 0 : 1] : a.rg_rows ? range_smem_bytes<VT>(a.rg_rows, a.rg_ext, a.rg_stage) : 0;
   // the instantiation of the form this matrix uses
   const int form = a.tri_cta ? TRI_CTA : a.rg_rows ? (A->tri.rg_k == 10 ? TRI_RANGE10 : TRI_RANGE7) : TRI_SYNCFREE;
-  if (method == EGPU_CG) return launch_cg(ctx, a, offs, form, smem);
+  if (method == EGPU_CG) return launch_cg(ctx, a, offs, form, smem, load);
   if constexpr (sizeof(VT) == 8) {
-    if (method == EGPU_GCR || method == EGPU_BICGSTABL) return launch_ext(ctx, a, method, form, smem);
+    if (method == EGPU_GCR || method == EGPU_BICGSTABL) return launch_ext(ctx, a, method, form, smem, load);
   }
-  return launch_bicgstab(ctx, a, offs, form, smem);
+  return launch_bicgstab(ctx, a, offs, form, smem, load);
 }
 
 // Loads the Krylov kernel a solve is about to launch (kernels are loaded on first use) without
@@ -1196,7 +1227,7 @@ static int krylov_load(egpu_mat *A, const egpu_params *prm, int sweeps) {
     a.sweeps_l = a.sweeps_u = sweeps;
     if (sweeps > 0) a.tri_cta = a.rg_rows = 0;
   }
-  return run_krylov<VT>(A, a, prm->method, A->sell_c16.p != nullptr);
+  return run_krylov<VT>(A, a, prm->method, A->sell_c16.p != nullptr, true);
 }
 
 // stored vectors of GCR (2 (m-1) directions) / BiCGStab(l) (r_0..r_l, u_0..u_l, shadow, x,

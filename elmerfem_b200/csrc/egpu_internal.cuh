@@ -132,7 +132,15 @@ struct egpu_ctx {
   unsigned int *sync_host_err = nullptr;
   // host-mapped abort word (egpu_abort): written by any host thread, polled by the kernels
   volatile int *abort_word = nullptr;
-  std::vector<const void *> shared_allowed;  // kernels this context has passed to allow_shared
+  // what this context has asked the runtime about its kernels: shared memory allowed
+  // (allow_shared), blocks an SM holds at the last size of shared memory (kernel_blocks)
+  struct KernelUse {
+    const void *kernel;
+    bool shared_allowed;
+    size_t smem;
+    int bps;  // 0: not asked yet
+  };
+  std::vector<KernelUse> kernel_uses;
 };
 
 // A copy between host and device memory in the order of the context's stream, complete on return.

@@ -3,21 +3,10 @@
 
 namespace egpu {
 
-int launch_ext(egpu_ctx *ctx, KArgs<double> &a, int method, int form, size_t smem) {
-  if (method == EGPU_GCR) {
-    switch (form) {
-      case TRI_CTA: return launch_coop(ctx, gcr_kernel<TRI_TS, TRI_CTA>, a, nullptr, smem);
-      case TRI_RANGE7: return launch_coop(ctx, gcr_kernel<TRI_TS, TRI_RANGE7>, a, nullptr, smem);
-      case TRI_RANGE10: return launch_coop(ctx, gcr_kernel<TRI_TS, TRI_RANGE10>, a, nullptr, smem);
-      default: return launch_coop(ctx, gcr_kernel<TRI_TS, TRI_SYNCFREE>, a, nullptr, smem);
-    }
-  }
-  switch (form) {
-    case TRI_CTA: return launch_coop(ctx, bicgstabl_kernel<TRI_TS, TRI_CTA>, a, nullptr, smem);
-    case TRI_RANGE7: return launch_coop(ctx, bicgstabl_kernel<TRI_TS, TRI_RANGE7>, a, nullptr, smem);
-    case TRI_RANGE10: return launch_coop(ctx, bicgstabl_kernel<TRI_TS, TRI_RANGE10>, a, nullptr, smem);
-    default: return launch_coop(ctx, bicgstabl_kernel<TRI_TS, TRI_SYNCFREE>, a, nullptr, smem);
-  }
+int launch_ext(egpu_ctx *ctx, KArgs<double> &a, int method, int form, size_t smem, bool load) {
+  if (method == EGPU_GCR)
+    return launch_form(ctx, a, form, smem, 0, load, [](auto tri) { return gcr_kernel<TRI_TS, decltype(tri)::value>; });
+  return launch_form(ctx, a, form, smem, 0, load, [](auto tri) { return bicgstabl_kernel<TRI_TS, decltype(tri)::value>; });
 }
 
 }  // namespace egpu

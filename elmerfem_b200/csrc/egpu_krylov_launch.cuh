@@ -1,9 +1,10 @@
-// egpu_krylov_launch.cuh -- launches of the persistent Krylov kernels.  Each method's kernels
-// are instantiated in a translation unit of their own (egpu_kcg.cu, egpu_kbicgstab.cu,
-// egpu_kext.cu).
+// egpu_krylov_launch.cuh -- launches of the persistent Krylov kernels.  The kernels of a method and
+// a precision are instantiated in a translation unit of their own (egpu_kcg32.cu, egpu_kcg64.cu,
+// egpu_kbicgstab32.cu, egpu_kbicgstab64.cu, egpu_kext.cu), so that they compile side by side.
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "egpu_krylov.cuh"
 #include "egpu_solve.h"
@@ -15,24 +16,16 @@ namespace egpu {
 // produce the value it waits for.
 constexpr int TRI_TS = 32;
 
-// occupancy-sized cooperative launch, of at most `most` blocks (0: no limit)
+// occupancy-sized cooperative launch, of at most `most` blocks (0: no limit); load: none, the
+// kernel is loaded only
 template <typename K, typename Args>
-int launch_coop(egpu_ctx *ctx, K kernel, Args &args, int *grid_out = nullptr, size_t smem = 0, int most = 0) {
+int launch_coop(egpu_ctx *ctx, K kernel, Args &args, size_t smem, int most, bool load) {
   int bps = 0;
-  if (smem > 48 * 1024) {
-    const int rc = allow_shared(ctx, (const void *)kernel);
-    if (rc) return rc;
-  }
-  EGPU_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, EGPU_KBLOCK, smem));
-  if (bps < 1) {
-    egpu_set_error(ctx, "persistent kernel does not fit on an SM");
-    return EGPU_ERR_CUDA;
-  }
-  if (args.nslices == 0) return EGPU_OK;  // the query above has loaded the kernel (krylov_load)
+  const int rc = kernel_blocks(ctx, (const void *)kernel, smem, &bps);
+  if (rc || load) return rc;
   bps = std::min(bps, 2048 / EGPU_KBLOCK);
   int grid = ctx->num_sms * bps;
   if (most > 0) grid = std::min(grid, most);
-  if (grid_out) *grid_out = grid;
   void *kargs[] = {&args};
   EGPU_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(EGPU_KBLOCK),
                                                  kargs, smem, ctx->stream));
@@ -49,11 +42,28 @@ inline int krylov_blocks(int nslices) {
   return std::max(1, (nslices + SLICES_PER_BLOCK - 1) / SLICES_PER_BLOCK);
 }
 
-// offs: 16-bit column offsets; form: a TriForm; smem: dynamic shared memory per block
-int launch_cg(egpu_ctx *ctx, KArgs<double> &a, bool offs, int form, size_t smem);
-int launch_cg(egpu_ctx *ctx, KArgs<float> &a, bool offs, int form, size_t smem);
-int launch_bicgstab(egpu_ctx *ctx, KArgs<double> &a, bool offs, int form, size_t smem);
-int launch_bicgstab(egpu_ctx *ctx, KArgs<float> &a, bool offs, int form, size_t smem);  // sweeps: a.sweeps_l > 0
-int launch_ext(egpu_ctx *ctx, KArgs<double> &a, int method, int form, size_t smem);     // GCR, BiCGStab(l)
+// pick(form as a constant): the kernel instantiated for that form; most: blocks without triangular
+// solves (0: no limit)
+template <typename VT, typename Pick>
+int launch_form(egpu_ctx *ctx, KArgs<VT> &a, int form, size_t smem, int most, bool load, Pick pick) {
+  switch (form) {
+    case TRI_CTA: return launch_coop(ctx, pick(std::integral_constant<int, TRI_CTA>{}), a, smem, 0, load);
+    case TRI_RANGE7: return launch_coop(ctx, pick(std::integral_constant<int, TRI_RANGE7>{}), a, smem, 0, load);
+    case TRI_RANGE10: return launch_coop(ctx, pick(std::integral_constant<int, TRI_RANGE10>{}), a, smem, 0, load);
+    default:
+      return launch_coop(ctx, pick(std::integral_constant<int, TRI_SYNCFREE>{}), a, smem,
+                         a.precond == EGPU_PREC_ILU0 ? 0 : most, load);
+  }
+}
+
+// offs: 16-bit column offsets; form: a TriForm; smem: dynamic shared memory per block; load: see
+// launch_coop
+int launch_cg(egpu_ctx *ctx, KArgs<double> &a, bool offs, int form, size_t smem, bool load);
+int launch_cg(egpu_ctx *ctx, KArgs<float> &a, bool offs, int form, size_t smem, bool load);
+int launch_bicgstab(egpu_ctx *ctx, KArgs<double> &a, bool offs, int form, size_t smem, bool load);
+// sweeps: a.sweeps_l > 0
+int launch_bicgstab(egpu_ctx *ctx, KArgs<float> &a, bool offs, int form, size_t smem, bool load);
+// GCR, BiCGStab(l)
+int launch_ext(egpu_ctx *ctx, KArgs<double> &a, int method, int form, size_t smem, bool load);
 
 }  // namespace egpu

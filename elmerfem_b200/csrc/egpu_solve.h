@@ -27,6 +27,7 @@ inline double inner_tol_of(const egpu_params *p) {
 
 int ensure_ctx_scratch(egpu_ctx *ctx);
 int allow_shared(egpu_ctx *ctx, const void *kernel);
+int kernel_blocks(egpu_ctx *ctx, const void *kernel, size_t smem, int *bps);
 int reset_sync(egpu_ctx *ctx);
 int scale_matrix(egpu_mat *A, bool scale_system, bool crs, bool f32);
 int ensure_ilu_structure(egpu_mat *A, int order);

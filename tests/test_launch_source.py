@@ -22,3 +22,13 @@ def test_shared_memory_limit_is_set_to_the_device_maximum_only():
     body = src[start:src.index("\n}", at)]
     assert "cudaDevAttrMaxSharedMemoryPerBlockOptin" in body and "sharedSizeBytes" in body
     assert "smem" not in body
+
+
+def test_loading_a_kernel_is_asked_for_by_an_argument():
+    """A launch whose arguments are not set fails or runs; it is never taken for a request to load only."""
+    with open(os.path.join(CSRC, "egpu_krylov_launch.cuh")) as f:
+        src = re.sub(r"//[^\n]*", "", f.read())
+    body = src[src.index("int launch_coop("):]
+    body = body[:body.index("\n}")]
+    assert "load" in body and "args." not in body
+    assert "cudaOccupancy" not in src  # asked once per context (kernel_blocks)
