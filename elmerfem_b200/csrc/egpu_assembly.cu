@@ -239,7 +239,7 @@ __device__ __forceinline__ double hex_point(const double *X, int t, int cdim, do
     }
   const double detG = G[0][0] * (G[1][1] * G[2][2] - G[1][2] * G[2][1]) + G[0][1] * (G[1][2] * G[2][0] - G[1][0] * G[2][2]) +
                       G[0][2] * (G[1][0] * G[2][1] - G[1][1] * G[2][0]);
-  const bool ok = detG > EGPU_TINY_DP;
+  const bool ok = !(detG <= EGPU_TINY_DP);  // NaN coordinates give NaN, not a missing element
   const double q = ok ? 1.0 / detG : 0.0;
   double GI[3][3];
   GI[0][0] = q * (G[1][1] * G[2][2] - G[2][1] * G[1][2]);
