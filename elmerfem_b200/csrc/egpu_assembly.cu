@@ -7,8 +7,7 @@
 // evaluate the geometry of one integration point each (ElementInfo / ElementMetric,
 // ElementDescription.src:2586-3320, 6757-6884) into shared memory, then all lanes form the
 // element matrix entries.  Entries are added to precomputed CRS positions.  Elements of one
-// colour share no node, so the scatter needs no atomics; the groups (a range of rows, then a
-// colour) run one after another.
+// colour share no node, so the scatter needs no atomics; colours run one after another.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -159,7 +158,6 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
 }
 
 constexpr int ASM_WARPS = 8;
-constexpr long long ASM_RANGE_BYTES = 40LL << 20;  // Values of one row range (see egpu_assembly_bind)
 
 // ------------------------------------------------------------------------------------
 // Hexahedra (808), four elements per warp.
@@ -177,7 +175,7 @@ constexpr long long ASM_RANGE_BYTES = 40LL << 20;  // Values of one row range (s
 //   3. per element: two gradients per lane, six (Poisson) or eighteen (elasticity) matrix
 //      instructions, and the accumulators are exactly the lane's CRS entries (two columns)
 // The CRS positions and the values they hold are loaded before step 2, so their latency is
-// covered by it.  Elements of a group share no node, so the preloaded values are current.
+// covered by it.  Elements of a colour share no node, so the preloaded values are current.
 constexpr int HEX_EPW = 4;       // elements per warp
 constexpr int HEX_XS = 25;       // doubles per element of staged coordinates (24 + 1: no bank conflicts)
 constexpr int HEX_LS = 12;       // doubles per point: L (9), weight, load weight, pad
@@ -752,27 +750,15 @@ extern "C" int egpu_assembly_bind(egpu_mat *A, int nnodes, const double *xyz, in
   }
   std::vector<int> color_of;
   const int ncol = egpu_color_elements(nnodes, nelem, nen, elem_nodes, color_of);
-  // Groups of elements assembled in one launch: a range of matrix rows, then a colour.  Every
-  // colour touches every row, so running each colour over the whole mesh would stream Values
-  // through HBM once per colour; a range whose Values fit in L2 (ASM_RANGE_BYTES of the 126 MB)
-  // is read and written there once for all its colours.
-  const long long nrange = std::max(1LL, (A->nnz * (long long)sizeof(double) + ASM_RANGE_BYTES / 2) / ASM_RANGE_BYTES);
-  const int nrows = A->n / dofs;
-  std::vector<int> group_of(nelem);
-  for (int e = 0; e < nelem; ++e) {
-    int lo = nrows - 1;
-    for (int k = 0; k < nen; ++k) {
-      const int r = p0[en0[(size_t)e * nen + k]];
-      if (r >= 0) lo = std::min(lo, r);
-    }
-    group_of[e] = (int)((long long)std::max(lo, 0) * nrange / std::max(1, nrows)) * ncol + color_of[e];
-  }
-  const int ngroup = (int)nrange * ncol;
-  S.color_ptr.assign(ngroup + 1, 0);
-  for (int e = 0; e < nelem; ++e) S.color_ptr[group_of[e] + 1]++;
-  for (int c = 0; c < ngroup; ++c) S.color_ptr[c + 1] += S.color_ptr[c];
+  // One launch per colour.  (Groups by row range and colour, so that a range's Values stay in L2 for
+  // all its colours, were slower at every size: hex 96^3 693 against 615 us, 128^3 1,591 and
+  // 1,362, elasticity 64^3 2,158 and 1,403, tetrahedral elasticity 56^3 3,350 and 3,018, and with
+  // elements in random order 4,265 and 1,648 at 64^3: a group is then one or two waves, bound by its own chain.)
+  S.color_ptr.assign(ncol + 1, 0);
+  for (int e = 0; e < nelem; ++e) S.color_ptr[color_of[e] + 1]++;
+  for (int c = 0; c < ncol; ++c) S.color_ptr[c + 1] += S.color_ptr[c];
   std::vector<int> grouped(nelem), fill(S.color_ptr.begin(), S.color_ptr.end() - 1);
-  for (int e = 0; e < nelem; ++e) grouped[fill[group_of[e]]++] = e;
+  for (int e = 0; e < nelem; ++e) grouped[fill[color_of[e]]++] = e;
   const int nd = nen * dofs;
   EGPU_CUDA_TRY(ctx, S.xyz.alloc((size_t)nnodes * 3));
   EGPU_CUDA_TRY(ctx, S.elem_nodes.alloc(en0.size()));
