@@ -95,6 +95,9 @@ __device__ __forceinline__ int batch_locate(const BatchShared &sh, int q) {
   return l;
 }
 
+// LISTS: the sum reads one offset list for a slice whose rows share it (slice_sum; it is short and
+// stays in L2), else every entry's offset (slice_spmv2)
+template <bool LISTS>
 __device__ __forceinline__ SliceMeta batch_slice_meta(const BatchArgs &ba, const BatchShared &sh, int q, int hi,
                                                       unsigned run) {
   SliceMeta m{nullptr, nullptr, 0u, 0u};
@@ -110,7 +113,7 @@ __device__ __forceinline__ SliceMeta batch_slice_meta(const BatchArgs &ba, const
   m.vals = d.svals + p;
   m.vbytes = (unsigned)(32 * w * (int)sizeof(float));
   if (d.scols16) {
-    if (__ldg(d.sell_cptr + sl) >= 0) {
+    if (!LISTS || __ldg(d.sell_cptr + sl) >= 0) {
       m.cols = d.scols16 + p;
       m.cbytes = (unsigned)(32 * w * (int)sizeof(int16_t));
     }
@@ -245,14 +248,14 @@ __device__ __forceinline__ void batch_spmv1(const BatchArgs &ba, const BatchShar
   const int total = sh.total, nb = gridDim.x;
   const int lo = (int)((long long)total * blockIdx.x / nb), hi = (int)((long long)total * (blockIdx.x + 1) / nb);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
-  SliceMeta next = batch_slice_meta(ba, sh, lo + warp + nw, hi, run);
+  SliceMeta next = batch_slice_meta<true>(ba, sh, lo + warp + nw, hi, run);
   for (int q = lo + warp; q < hi; q += nw) {
     const int a = batch_locate(sh, q);
     if (lane == 0 && next.vbytes) {
       prefetch_l2_bulk(next.vals, next.vbytes);
       if (next.cbytes) prefetch_l2_bulk(next.cols, next.cbytes);
     }
-    next = batch_slice_meta(ba, sh, q + 2 * nw, hi, run);
+    next = batch_slice_meta<true>(ba, sh, q + 2 * nw, hi, run);
     const int s = sh.act[a];
     if (!((run >> sh.status[s]) & 1u)) continue;
     const int slice = q - sh.pre[a];
@@ -268,8 +271,8 @@ __device__ __forceinline__ void batch_spmv2(const BatchArgs &ba, const BatchShar
   const int lo = (int)((long long)total * blockIdx.x / nb), hi = (int)((long long)total * (blockIdx.x + 1) / nb);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int g = ba.spw == 2 ? 2 : 1, step = g * nw;  // slices a warp takes at once, and its stride
-  SliceMeta n0 = batch_slice_meta(ba, sh, lo + warp + step, hi, run),
-            n1 = batch_slice_meta(ba, sh, g == 2 ? lo + warp + step + nw : hi, hi, run);
+  SliceMeta n0 = batch_slice_meta<false>(ba, sh, lo + warp + step, hi, run),
+            n1 = batch_slice_meta<false>(ba, sh, g == 2 ? lo + warp + step + nw : hi, hi, run);
   for (int q0 = lo + warp; q0 < hi; q0 += step) {
     const int q1 = g == 2 ? q0 + nw : hi;
     if (lane == 0) {
@@ -282,8 +285,8 @@ __device__ __forceinline__ void batch_spmv2(const BatchArgs &ba, const BatchShar
         if (n1.cbytes) prefetch_l2_bulk(n1.cols, n1.cbytes);
       }
     }
-    n0 = batch_slice_meta(ba, sh, q0 + 2 * step, hi, run);
-    n1 = batch_slice_meta(ba, sh, g == 2 ? q1 + 2 * step : hi, hi, run);
+    n0 = batch_slice_meta<false>(ba, sh, q0 + 2 * step, hi, run);
+    n1 = batch_slice_meta<false>(ba, sh, g == 2 ? q1 + 2 * step : hi, hi, run);
     const int a0 = batch_locate(sh, q0), s0 = sh.act[a0], sl0 = q0 - sh.pre[a0];
     int a1 = -1, s1 = 0, sl1 = 0;
     if (q1 < hi) {
