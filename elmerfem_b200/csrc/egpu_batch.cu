@@ -1260,8 +1260,9 @@ __device__ __forceinline__ void team_vec(int r0, int r1, F &&f) {
 }
 
 // A lane's row sum, U entries at a time.  The unrolling should divide the row: what is left over
-// after the last whole chunk goes one entry, two round trips, at a time.  5 for the tets' 15
-// entries, 9 for 27-point rows (96 tet systems: 16 82 ms, 15 54 ms, 5 52 ms).
+// after the last whole chunk goes one entry, two round trips, at a time.  9 for 27-point rows, 8
+// for rows of 8, 16 and 24 (148 systems of 20,000 rows, 40 iterations: 8 entries by 5 123 ms, by 8
+// 104; 24 entries 237 and 226), else 5, the tets' 15 entries (96 tet systems: 16 82 ms, 15 54, 5 52).
 template <int U>
 __device__ __forceinline__ float team_row(const TeamSys &S, const float *P, int r, int base, int w) {
   float t = 0.f;
@@ -1383,8 +1384,10 @@ __device__ bool team_solve(const TeamArgs &a, const TeamSys &S, int rank, TeamOu
             const int e = base + (kk << 5);
             t = fmaf(__ldcs(S.svals32 + e), __ldca(P + __ldcs(S.scols + e)), t);
           }
-        } else if (w % 9) {
+        } else if (w % 9 && w % 8) {
           t = team_row<5>(S, P, r, base, w);
+        } else if (w % 9) {
+          t = team_row<8>(S, P, r, base, w);
         } else {
           t = team_row<9>(S, P, r, base, w);
         }

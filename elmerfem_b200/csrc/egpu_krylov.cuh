@@ -202,9 +202,13 @@ __device__ __forceinline__ VT ld_l2(const VT *p) {
 // and a valid column.  epi(row, s0, s1) runs once per row on its own lane.
 //
 // The loops take U entries at a time, loads first; what is left over at the end of a row goes one
-// entry, two round trips, at a time, so U should divide the row: 9 for 27-point rows and 27-point
-// blocks (128^3 mixed CG's inner solves: 8 34.9 ms, 9 31.8 ms, 14 44.3, 27 37.0), else 5, the
-// tets' 15 entries (tet cube 40 mixed CG: 8 3.25 ms, 5 2.96 ms; hex at 5 35.2 ms).
+// entry, two round trips, at a time, so U is the one of 9, 8 and 5 with the fewest trips: 9 for
+// 27-point rows (128^3 mixed CG's inner solves: 8 34.9 ms, 9 31.8 ms, 14 44.3, 27 37.0), 5 for
+// the tets' 15 entries (tet cube 40 mixed CG: 8 3.25 ms, 5 2.96 ms), 8 for 8, 16, 24 and 32.  For
+// rows with offsets of their own the choice is by divisibility alone, which is as good there
+// and leaves the loops cheaper.  40 CG iterations in FP32 on 10^6 rows, U = 9 or 5 only and now:
+// rows that share their offsets, 7 entries 2.32 and 2.07 ms, 8 2.00 and 1.60, 15 2.85 and 2.70, 16
+// 2.70 and 2.36, 24 3.21 and 2.91; own offsets, 8 1.92 and 1.71, 16 2.45 and 2.38, 24 3.31 and 3.06.
 template <typename VT, int LPR, bool OFFS, bool TWO, typename F>
 __device__ __forceinline__ void spmv_phase(const KArgs<VT> &a, const VT *x0, const VT *x1, F &&epi) {
   const int lane = threadIdx.x & 31;
@@ -237,32 +241,41 @@ __device__ __forceinline__ void spmv_phase(const KArgs<VT> &a, const VT *x0, con
         for (int k0 = 0; k0 < w; k0 += 32) {
           const int kn = min(32, w - k0);
           const int offl = lane < kn ? (int)__ldg(co + k0 + lane) : 0;
-#pragma unroll 9
-          for (int k = 0; k < kn; ++k) {
+          auto shared_entry = [&](int k) {
             const VT v = ld_stream(a.svals + base + ((k0 + k) << 5));
             const int c = r + __shfl_sync(0xffffffffu, offl, k);
             s0 = row_madd(s0, v, ld_l2(x0 + c));
             if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
+          };
+          const int t9 = kn / 9 + kn % 9, t8 = kn / 8 + kn % 8, t5 = kn / 5 + kn % 5;
+          if (t9 <= t8 && t9 <= t5) {
+#pragma unroll 9
+            for (int k = 0; k < kn; ++k) shared_entry(k);
+          } else if (t8 <= t5) {
+#pragma unroll 8
+            for (int k = 0; k < kn; ++k) shared_entry(k);
+          } else {
+#pragma unroll 5
+            for (int k = 0; k < kn; ++k) shared_entry(k);
           }
         }
       } else {
         const int16_t *co = a.scolsc + cp + lane;
-        if (w % 9) {
+        auto own_entry = [&](int k) {
+          const VT v = ld_stream(a.svals + base + (k << 5));
+          const int c = r + (int)ld_stream(co + (k << 5));
+          s0 = row_madd(s0, v, ld_l2(x0 + c));
+          if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
+        };
+        if (w % 9 && w % 8) {
 #pragma unroll 5
-          for (int k = 0; k < w; ++k) {
-            const VT v = ld_stream(a.svals + base + (k << 5));
-            const int c = r + (int)ld_stream(co + (k << 5));
-            s0 = row_madd(s0, v, ld_l2(x0 + c));
-            if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
-          }
+          for (int k = 0; k < w; ++k) own_entry(k);
+        } else if (w % 9) {
+#pragma unroll 8
+          for (int k = 0; k < w; ++k) own_entry(k);
         } else {
 #pragma unroll 9
-          for (int k = 0; k < w; ++k) {
-            const VT v = ld_stream(a.svals + base + (k << 5));
-            const int c = r + (int)ld_stream(co + (k << 5));
-            s0 = row_madd(s0, v, ld_l2(x0 + c));
-            if (TWO) s1 = row_madd(s1, v, ld_l2(x1 + c));
-          }
+          for (int k = 0; k < w; ++k) own_entry(k);
         }
       }
     } else {
