@@ -1287,8 +1287,8 @@ __device__ bool team_solve(const TeamArgs &a, const TeamSys &S, int rank, TeamOu
   int refinements = 0, inner_total = 0, info = 0, last_info = 0;
   double residual = 0.0, rnorm = 1.0, rnorm_prev = 1.0, carry_rho = 0.0;
   while (true) {
-    // cancellation: the host-mapped abort word, read once per refinement (the barrier of the
-    // residual's sum below then takes every member out)
+    // cancellation: the host-mapped abort word, read once per refinement (the next barriers take
+    // every member out: at once with several CTAs, within TEAM_ERR_EVERY barriers with one)
     if (threadIdx.x == 0) egpu_poll_abort(a.err);
     // ---- FP64 residual r = bs - A xs on this member's rows (as k_batch_residual)
     double acc[2] = {0.0, 0.0};

@@ -30,7 +30,7 @@ enum TriForm { TRI_SYNCFREE = 0, TRI_CTA, TRI_RANGE7, TRI_RANGE10 };
 constexpr bool tri_range(int form) { return form == TRI_RANGE7 || form == TRI_RANGE10; }
 
 // One triangle of the row-range solve on the device: the level records of every range
-// (plan::range_records, with values), slot of every row, external rows
+// (laid out by plan::range_record, with values), slot of every row, external rows
 struct RangeTri {
   const int *lev_ptr;
   const long long *offset;
@@ -586,8 +586,9 @@ __device__ __forceinline__ void upper_solve_blk(const KArgs<VT> &a, const VT *y,
 // level costs a store, an L2 round trip, a poll and a warp's sum (0.9 us; 1.7 us for a node
 // block).  Here a block owns a contiguous range of rows, whose values it keeps in shared memory
 // and solves level by level, one block barrier a level: G lanes a row, K entries a lane, all of
-// a level's rows at once, the entries staged by one bulk copy a level.  Only dependencies that cross a range boundary go through L2, and
-// those are off the chain: separate warps fetch them into shared memory as they are published.
+// a level's rows at once, the entries staged by one bulk copy a level.  Every value is published
+// to global memory, and the ones another range's rows read are fetched from L2 into its shared
+// memory by separate warps, off the chain of levels.
 // (A warp per row polling shared memory was slower than no ranges at all: the polls of the
 // waiting warps take the issue slots and the shared-memory pipe from the warp on the chain.)
 //

@@ -1,4 +1,5 @@
-// egpu_tri_cta.cu -- host side of the level-synchronous single-block ILU0 solves.
+// egpu_tri_cta.cu -- host side of the level-synchronous single-block ILU0 solves and of the
+// row-range solves (second half of the file; plan in egpu_tri_range.h).
 //
 // The sync-free solves (egpu_krylov.cuh) spread a level over the whole GPU and pay a
 // cross-SM publish/observe round trip per dependency level.  On meshes whose levels are

@@ -150,8 +150,8 @@ inline double range_cycles(int n, int bs, int per, RangeShape sh, int ext, bool 
   return cycles;
 }
 
-// The plan of one triangle; false when it does not fit (node blocks of unequal columns, or more
-// shared-memory cells than 16-bit indices reach).  zero: index of a cell holding 0 (padding).
+// The plan of one triangle; false when it does not fit (a row with more entries than its lanes
+// hold, or more shared-memory cells than 16-bit indices reach).
 inline bool range_triangle(int n, int bs, int per, RangeShape sh, bool lower, const std::vector<int> &rows,
                            const std::vector<int> &cols, const std::vector<int> &diag, const std::vector<int> &lev,
                            RangeTriHost &T) {
